@@ -99,3 +99,27 @@ def test_container_columns_decode_on_gpu(cuda, tmp_path):
     want = int(vals.view(np.uint32).astype(np.uint64).sum())
     assert int(ops.query_aggregate(g2.to_device()).cpu()[0]) & 0xFFFFFFFFFFFFFFFF == want
     ops.check_device_error()
+
+
+@pytest.mark.parametrize("bits", [0, 1, 9, 21, 22, 23, 31, 32])
+@pytest.mark.parametrize("n_distinct", [1, 2, 255, 1023, 1024])
+def test_gpu_encoder_dictionary_ranges(cuda, bits, n_distinct):
+    """Dictionaries around the widest range whose sort keys carry the value's
+    index (22 bits), from one distinct value to all 1024, in both layouts."""
+    g = np.random.default_rng(bits * 1024 + n_distinct)
+    lo, n = -(1 << 31) if bits == 32 else -12345, min(n_distinct, 1 << bits)
+    pool = lo + np.unique(np.concatenate([[0, (1 << bits) - 1], g.integers(0, 1 << bits, 4 * n, dtype=np.int64)]))
+    pool = np.concatenate([[pool[0], pool[-1]], g.permutation(pool[1:-1])])[:n]
+    vals = np.concatenate([g.permutation(np.resize(pool, 1024)) for _ in range(9)] + [pool[:1]]).astype(np.int32)
+    for layout in (LAYOUT_NORMAL, LAYOUT_TRANSPOSED):
+        _compare(vals, 4, layout)
+
+
+@pytest.mark.parametrize("n_vec", [7, 8, 9, 8 * 32 + 1, 8 * 128, 8 * 128 + 8, 8 * 129 + 3, 8 * 1500 + 5])
+def test_gpu_encoder_offsets_over_many_tiles(cuda, n_vec):
+    """Offsets, total, largest vector and scheme mask around the look-back's
+    window (128 tiles of 8 vectors) and past the resident CTAs."""
+    g = np.random.default_rng(n_vec)
+    vals = (g.integers(0, 1 << 31, (n_vec, 1024)) >> g.integers(0, 31, (n_vec, 1))).astype(np.int32).reshape(-1)[:-11]
+    schemes = np.where(g.integers(0, 50, n_vec) == 0, g.integers(0, 5, n_vec), 0).astype(np.uint8)
+    _compare(vals, schemes, LAYOUT_TRANSPOSED)
