@@ -7,8 +7,9 @@
 // without leaving the device.  One kernel reads the values once: a CTA takes
 // tiles of eight consecutive vectors in order; one warp per vector stages its
 // 1024 values in shared memory and computes the chosen scheme's bit width, aux
-// and payload words; the tile's word offset comes from a look-back over the
-// tiles before it; the warp then writes the payload it still holds.
+// and payload words; a warp of one more CTA adds up the tiles' words in order
+// and answers with each tile's offset; the warp then writes the payload it
+// still holds.
 //
 // Layout facts restated from the reference: the lane/word order of
 // fastlanes/src/pack.cpp:1954-1990, the transposed order of
@@ -19,16 +20,23 @@
 
 #include <algorithm>
 
-#include "fls_pipeline.cuh"
+#include "fls_selector.cuh"
 
 namespace fls {
 namespace {
 
 constexpr uint32_t kEncWarps    = 8;                 // warps per CTA
-constexpr uint32_t kValWords    = 33u * 32u;         // the vector, 33-padded rows
-constexpr uint32_t kEncWarpWords = 2u * kValWords;   // the vector; sort buffer, then dictionary
+// A warp's shared memory, in words: the staged vector (33-padded), which is
+// also the sort's buffer; in its place afterwards a DICT vector's 16-bit codes
+// (34-padded) and its dictionary, or an RLE vector's run values; past the
+// staged vector, before that, the statistics' buckets and the network's
+// activations.
+constexpr uint32_t kCodeWords    = 34u * 32u / 2u;
+constexpr uint32_t kEncWarpWords = kCodeWords + 1024u;
+constexpr uint32_t kNetWords     = sel::kPadded + sel::kBuckets / 4u; // offset of the activations
+static_assert(kEncWarpWords % 4 == 0 && kEncWarpWords >= kNetWords + sel::WarpNet::kScratch, "the warp's words");
 constexpr uint32_t kKeyedBits    = 22;               // widest range whose sort keys carry the value's index
-constexpr uint32_t kPollLimit   = 1u << 22;          // bounded look-back waits (each poll is an L2 round trip)
+constexpr uint32_t kPollLimit   = 1u << 22;          // bounded waits on other tiles (each poll is an L2 round trip)
 
 struct EncParams {
 	const int32_t* values;
@@ -42,30 +50,29 @@ struct EncParams {
 	uint32_t*      out;
 	fls_vec_meta*  meta;
 	uint64_t       n_tiles;
-	uint32_t*      counter; // next tile to take (zeroed before the launch)
-	uint64_t*      tiles;   // per tile: look-back state (zeroed before the launch)
-	uint64_t*      info;    // [0] total words, [1] max vector words, [2] scheme mask
+	uint32_t*      counter; // next ticket, CTAs done (zeroed before the launch)
+	uint64_t*      reports; // per tile (zeroed before the launch)
+	uint64_t*      offsets; // per tile (zeroed before the launch)
+	uint64_t*      info;    // [0] total words, [1] max vector words, [2] scheme mask; learned: [3] fallbacks
 	uint32_t*      err;
+	// learned selection
+	const float*        params;
+	float               threshold;
+	double              kappa;
+	uint8_t*            picks;      // the chosen scheme per vector, or null
+	unsigned long long* n_fallback; // vectors below the threshold (zeroed before the launch)
 };
 
-// Look-back state of a tile, one 64-bit word: payload words (42 bits: at most
-// 2^30 vectors of kMaxVecWords), largest vector (11 bits), scheme mask (5
-// bits), and a flag: not there yet, of the tile alone, of all tiles up to it,
-// or given up.
-constexpr uint64_t kTileSum = (1ull << 42) - 1ull, kTileBody = (1ull << 62) - 1ull;
-constexpr uint64_t kTileOwn = 1ull << 62, kTileAll = 2ull << 62, kTileLost = 3ull << 62;
-static_assert(kMaxVecWords < (1u << 11) && FLS_N_SCHEMES <= 5 && FLS_MAX_VALUES / 1024u * kMaxVecWords <= kTileSum,
-              "look-back state fields");
+// What a tile reports, one 64-bit word: its payload words (low half), its
+// largest vector (16 bits), its scheme mask (8 bits) and a mark that it is
+// there.  What it gets back: its word offset and the mark, or kTileLost.
+constexpr uint64_t kTileMark = 1ull << 63, kTileLost = ~0ull;
+static_assert(kMaxVecWords < (1u << 16) && FLS_N_SCHEMES <= 8 && FLS_MAX_VALUES / 1024u * kMaxVecWords < kTileMark,
+              "tile report fields");
 
-__device__ __forceinline__ uint64_t tile_state(uint64_t words, uint32_t max_words, uint32_t mask) {
-	return words | (static_cast<uint64_t>(max_words) << 42) | (static_cast<uint64_t>(mask) << 53);
+__device__ __forceinline__ uint64_t tile_report(uint32_t words, uint32_t max_words, uint32_t mask) {
+	return kTileMark | (static_cast<uint64_t>(mask << 16 | max_words) << 32) | words;
 }
-__device__ __forceinline__ uint32_t tile_max(uint64_t s) { return static_cast<uint32_t>(s >> 42) & 0x7ffu; }
-__device__ __forceinline__ uint32_t tile_mask(uint64_t s) { return static_cast<uint32_t>(s >> 53) & 0x1fu; }
-__device__ __forceinline__ uint64_t tile_join(uint64_t a, uint64_t b) {
-	return tile_state((a & kTileSum) + (b & kTileSum), max(tile_max(a), tile_max(b)), tile_mask(a) | tile_mask(b));
-}
-
 __device__ __forceinline__ uint64_t tile_load(const uint64_t* p) {
 	uint64_t v;
 	asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -75,66 +82,64 @@ __device__ __forceinline__ void tile_store(uint64_t* p, uint64_t v) {
 	asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// One warp: the joined state of all tiles before `tile` (no flag), after
-// publishing this tile's own; kTileLost when a wait gave up (the bound is
-// never met by a running grid: tiles are taken in order, so every tile before
-// this one belongs to a resident CTA).  A round reads kLookGroups x 32 tiles,
-// all loads in flight: tiles finish at one window per L2 round trip at most,
-// so a window of 32 tiles held a large column to 1.5 TB/s of values (it
-// measured 0.90-0.97x of separate plan, scan and write kernels).
-constexpr uint32_t kLookGroups = 4;
-__device__ __forceinline__ uint64_t tile_lookback(uint64_t* tiles, uint64_t tile, uint64_t own, uint32_t lane) {
-	if (tile == 0) {
-		if (lane == 0) { tile_store(tiles, own | kTileAll); }
-		return 0;
-	}
-	if (lane == 0) { tile_store(tiles + tile, own | kTileOwn); }
-	uint64_t before = 0;
-	for (uint64_t end = tile;;) { // tiles [0, end) are still to be joined
-		uint64_t s[kLookGroups];
-		uint32_t take[kLookGroups]; // lanes joined from each group
-		bool     got = false, done = false, lost = false;
-		for (uint32_t poll = 0; poll < kPollLimit && !got; ++poll) {
+// One warp: takes the tiles' reports in order, answers each with its offset
+// and leaves the column's totals in info.  A round reads kScanGroups x 32
+// reports, all loads in flight, and answers those that are there.  Tiles are
+// taken in order by running CTAs, so the next report always comes; should
+// kPollLimit rounds bring none, the tiles still waiting are told so.
+//
+// Why one warp: a look-back by every tile over those before it (256 reports
+// per round trip) cost the tiles 4-7 us each on a column of 733 tiles, since
+// all of a GPU's tiles finish planning together and walk the same states.
+constexpr uint32_t kScanGroups = 8;
+__device__ void scan_tiles(const uint64_t* reports, uint64_t* offsets, uint64_t n_tiles, uint64_t* info, uint32_t* err,
+                           uint32_t lane) {
+	uint64_t pos = 0, run = 0;
+	uint32_t mx = 0, mask = 0, idle = 0;
+	while (pos < n_tiles) {
+		uint64_t s[kScanGroups];
 #pragma unroll
-			for (uint32_t g = 0; g < kLookGroups; ++g) {
-				const uint32_t back = 32u * g + lane;
-				s[g]                = back < end ? tile_load(tiles + (end - 1u - back)) : kTileAll;
+		for (uint32_t g = 0; g < kScanGroups; ++g) {
+			const uint64_t t = pos + 32u * g + lane;
+			s[g]             = t < n_tiles ? tile_load(reports + t) : 0ull;
+		}
+		const uint64_t pos0 = pos;
+		bool           more = true;
+#pragma unroll
+		for (uint32_t g = 0; g < kScanGroups; ++g) {
+			if (!more) { continue; }
+			const uint32_t none = __ballot_sync(0xffffffffu, s[g] == 0ull);
+			const uint32_t n    = none ? static_cast<uint32_t>(__ffs(none)) - 1u : 32u;
+			const bool     mine = lane < n;
+			const uint32_t hi   = mine ? static_cast<uint32_t>(s[g] >> 32) & 0x7fffffffu : 0u;
+			const uint32_t w    = mine ? static_cast<uint32_t>(s[g]) : 0u;
+			uint32_t       incl = w; // at most 32 tiles x 8 vectors of kMaxVecWords
+#pragma unroll
+			for (int o = 1; o < 32; o <<= 1) {
+				const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+				if (lane >= static_cast<uint32_t>(o)) { incl += y; }
 			}
-			got  = true;
-			done = false;
-#pragma unroll
-			for (uint32_t g = 0; g < kLookGroups; ++g) {
-				const uint64_t flag = s[g] & ~kTileBody;
-				const uint32_t all  = __ballot_sync(0xffffffffu, flag >= kTileAll);
-				const uint32_t none = __ballot_sync(0xffffffffu, flag == 0);
-				take[g]             = done ? 0u : all ? all ^ (all - 1u) : 0xffffffffu; // up to the first that knows all
-				got                 = got && (none & take[g]) == 0;
-				done                = done || all != 0;
-			}
+			if (mine) { tile_store(offsets + pos + lane, kTileMark | (run + incl - w)); }
+			run += __shfl_sync(0xffffffffu, incl, 31);
+			mx = max(mx, hi & 0xffffu);
+			mask |= hi >> 16;
+			pos += n;
+			more = n == 32u;
 		}
-		uint64_t sum = 0;
-		uint32_t mx = 0, mask = 0;
-#pragma unroll
-		for (uint32_t g = 0; g < kLookGroups; ++g) {
-			const bool mine = (take[g] >> lane) & 1u;
-			lost            = lost || (mine && (s[g] & ~kTileBody) == kTileLost);
-			const uint64_t b = mine ? s[g] & kTileBody : 0ull;
-			sum += b & kTileSum;
-			mx = max(mx, tile_max(b));
-			mask |= tile_mask(b);
+		idle = pos == pos0 ? idle + 1u : 0u;
+		if (idle == kPollLimit) {
+			if (lane == 0) { atomicOr(err, kErrTimeout); }
+			for (uint64_t t = pos + lane; t < n_tiles; t += 32u) { tile_store(offsets + t, kTileLost); }
+			return;
 		}
-		if (!got || __any_sync(0xffffffffu, lost)) {
-			if (lane == 0) { tile_store(tiles + tile, kTileLost); }
-			return kTileLost;
-		}
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) { sum += __shfl_xor_sync(0xffffffffu, sum, o); }
-		before = tile_join(before, tile_state(sum, __reduce_max_sync(0xffffffffu, mx), __reduce_or_sync(0xffffffffu, mask)));
-		if (done) { break; } // also at the column's start: tiles before it count as known
-		end -= 32u * kLookGroups;
 	}
-	if (lane == 0) { tile_store(tiles + tile, tile_join(before, own) | kTileAll); }
-	return before;
+	mx   = __reduce_max_sync(0xffffffffu, mx);
+	mask = __reduce_or_sync(0xffffffffu, mask);
+	if (lane == 0) {
+		info[0] = run;
+		info[1] = mx;
+		info[2] = mask;
+	}
 }
 
 __device__ __forceinline__ uint32_t bits_of(uint32_t v) { return v ? 32u - __clz(v) : 0u; }
@@ -152,47 +157,6 @@ __device__ __forceinline__ uint32_t payload_words(uint32_t scheme, uint32_t bw, 
 	case FLS_SCHEME_CONST: return 0u;
 	default: return 32u * bits_of(aux - 1u) + round_words4((aux * bw + 31u) / 32u); // DICT
 	}
-}
-
-// Loads vector v (the last one padded with the column's last value, as the
-// host encoder pads) into shared memory; returns this lane's min and max.
-__device__ __forceinline__ void stage_vector(const EncParams& P, uint64_t v, int32_t* sv, uint32_t lane, int32_t& mn,
-                                             int32_t& mx) {
-	const int32_t last = __ldg(P.values + (P.n - 1));
-	mn                 = INT32_MAX;
-	mx                 = INT32_MIN;
-	const uint64_t v0  = v * 1024u;
-	if (v0 + 1024u <= P.n && (reinterpret_cast<uintptr_t>(P.values) & 15u) == 0) { // warp-uniform
-		// a whole vector from a 16-byte aligned column: eight 16-byte loads
-		// per lane (values 128 k + 4 lane .. + 3), all in flight at once
-		int4 q[8];
-#pragma unroll
-		for (uint32_t k = 0; k < 8; ++k) { q[k] = __ldg(reinterpret_cast<const int4*>(P.values + v0) + 32u * k + lane); }
-		asm volatile("" ::: "memory"); // every load issued before the first store below
-#pragma unroll
-		for (uint32_t k = 0; k < 8; ++k) {
-			const uint32_t j = 128u * k + 4u * lane; // conflict-free: (j + j / 32) mod 32 differs across lanes
-			const int32_t  e[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
-#pragma unroll
-			for (uint32_t t = 0; t < 4; ++t) {
-				sv[(j + t) + ((j + t) >> 5)] = e[t];
-				mn                           = min(mn, e[t]);
-				mx                           = max(mx, e[t]);
-			}
-		}
-	} else {
-#pragma unroll 4
-		for (uint32_t r = 0; r < 32; ++r) {
-			const uint64_t idx = v0 + 32u * r + lane;
-			const int32_t  x   = idx < P.n ? __ldg(P.values + idx) : last;
-			sv[33u * r + lane] = x;
-			mn                 = min(mn, x);
-			mx                 = max(mx, x);
-		}
-	}
-	__syncwarp();
-	mn = __reduce_min_sync(0xffffffffu, mn);
-	mx = __reduce_max_sync(0xffffffffu, mx);
 }
 
 __device__ __forceinline__ void order(uint32_t& a, uint32_t& b) {
@@ -216,8 +180,8 @@ __device__ __forceinline__ void order_step(uint32_t (&k)[32]) {
 // way of buf (33-padded, conflict-free) so that lane L holds elements L, L +
 // 32, ...  A block that sorts downwards holds its keys complemented, so every
 // step is one min and one max.  About 2500 instructions per vector, against
-// 12000 for the same network on shared memory (low-cardinality dictionary of
-// 6 M values, whole encoder call: 308 -> 126 us).
+// 12000 for the same network on shared memory (6 M values as a dictionary,
+// whole encoder call: 308 -> 126 us).
 __device__ __forceinline__ void sort1024(uint32_t (&k)[32], uint32_t* buf, uint32_t lane) {
 	uint32_t flip = 0u - (lane & 1u);
 #pragma unroll
@@ -262,9 +226,10 @@ __device__ __forceinline__ void sort1024(uint32_t (&k)[32], uint32_t* buf, uint3
 
 // Sorts the staged vector's values minus mn (range bits rbw) into k, each
 // with its index below it when both fit 32 bits, and returns the number of
-// distinct values; first: the registers that hold the first of a value.
-__device__ __forceinline__ uint32_t sort_distinct(const int32_t* sv, uint32_t* buf, uint32_t lane, int32_t mn,
-                                                  uint32_t rbw, uint32_t (&k)[32], uint32_t& first, uint32_t& before) {
+// distinct values; first: the registers that hold the first of a value, of
+// which `before` are on lower lanes.  The staged vector is lost.
+__device__ __forceinline__ uint32_t sort_distinct(int32_t* sv, uint32_t lane, int32_t mn, uint32_t rbw,
+                                                  uint32_t (&k)[32], uint32_t& first, uint32_t& before) {
 	const bool     keyed = rbw <= kKeyedBits;
 	const uint32_t sh    = keyed ? 10u : 0u;
 #pragma unroll
@@ -273,7 +238,7 @@ __device__ __forceinline__ uint32_t sort_distinct(const int32_t* sv, uint32_t* b
 		k[r]             = keyed ? (d << 10) | (32u * lane + r) : d;
 	}
 	__syncwarp();
-	sort1024(k, buf, lane);
+	sort1024(k, reinterpret_cast<uint32_t*>(sv), lane);
 	const uint32_t last = __shfl_up_sync(0xffffffffu, k[31], 1);
 	first               = lane == 0 || ((k[0] ^ last) >> sh) != 0u ? 1u : 0u;
 #pragma unroll
@@ -289,15 +254,15 @@ __device__ __forceinline__ uint32_t sort_distinct(const int32_t* sv, uint32_t* b
 	return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// Dictionary of the sorted keys: the distinct values minus mn, ascending, in
-// u; with keys that carry the index, also the code of every value over the
-// staged vector (16-bit, 34-padded rows of 32).
+// Dictionary of the sorted keys: the distinct values minus mn, ascending, and,
+// with keys that carry the index, the code of every value.
 __device__ __forceinline__ uint16_t* codes_of(int32_t* sv) { return reinterpret_cast<uint16_t*>(sv); }
+__device__ __forceinline__ uint32_t* dict_of(int32_t* sv) { return reinterpret_cast<uint32_t*>(sv) + kCodeWords; }
 __device__ __forceinline__ uint32_t  code_pos(uint32_t j) { return j + 2u * (j >> 5); }
 
 __device__ __forceinline__ void write_dict(const uint32_t (&k)[32], uint32_t first, uint32_t before, bool keyed,
-                                           int32_t* sv, uint32_t* u) {
-	uint32_t n = before;
+                                           int32_t* sv) {
+	uint32_t *u = dict_of(sv), n = before;
 #pragma unroll
 	for (uint32_t r = 0; r < 32; ++r) {
 		const bool f = (first >> r) & 1u;
@@ -361,14 +326,32 @@ __device__ __forceinline__ void pack_sequential(const uint32_t* u, uint32_t n, u
 	if (bw == 0) { return; }
 	const uint32_t words = round_words4((n * bw + 31u) / 32u);
 	const uint32_t inv   = 0xffffffffu / bw + 1u; // bw == 1: 0
+	const uint32_t n_bits = n * bw;
+	if (bw >= 11) {
+		// a word meets at most four entries: read without a loop, so that the
+		// reads of several words are in flight together (past the last entry
+		// whatever lies there, masked off)
+#pragma unroll 4
+		for (uint32_t w = lane; w < words; w += 32) {
+			const uint32_t bit0 = 32u * w, k0 = __umulhi(bit0, inv), s0 = bit0 - k0 * bw;
+			uint32_t       word = u[min(k0, 1023u)] >> s0;
+#pragma unroll
+			for (uint32_t i = 1; i < 4; ++i) {
+				const uint32_t s = i * bw - s0, e = u[min(k0 + i, 1023u)];
+				word |= s < 32u ? e << s : 0u;
+			}
+			const uint32_t left = bit0 < n_bits ? n_bits - bit0 : 0u;
+			out[w]              = left < 32u ? word & ((1u << left) - 1u) : word;
+		}
+		return;
+	}
 	for (uint32_t w = lane; w < words; w += 32) {
 		const uint32_t bit0 = 32u * w;
-		const uint32_t k0   = bw == 1u ? bit0 : __umulhi(bit0, inv);
-		uint32_t       word = 0;
-		if (k0 < n) {
-			word = u[k0] >> (bit0 - k0 * bw);
-			uint32_t k = k0 + 1u;
-			for (uint32_t sh = (k0 + 1u) * bw - bit0; sh < 32u && k < n; sh += bw) { word |= u[k++] << sh; }
+		uint32_t       k    = bw == 1u ? bit0 : __umulhi(bit0, inv), word = 0;
+		if (k < n) {
+			uint32_t sh = (k + 1u) * bw - bit0;
+			word        = u[k++] >> (bw - sh);
+			for (; sh < 32u && k < n; sh += bw) { word |= u[k++] << sh; }
 		}
 		out[w] = word;
 	}
@@ -379,139 +362,105 @@ struct Plan {
 	int32_t  base;
 };
 
-// Scheme parameters of the staged vector (CONST on a non-constant vector
-// becomes FOR, as on the host).
-__device__ __forceinline__ Plan plan_vector(const EncParams& P, uint64_t v, int32_t* sv, uint32_t* u, uint32_t lane,
-                                            int32_t mn, int32_t mx) {
-	uint32_t s = P.schemes ? P.schemes[v] : P.scheme;
-	if (s >= FLS_N_SCHEMES) {
-		if (lane == 0) { atomicOr(P.err, kErrBadMeta); }
-		s = FLS_SCHEME_FOR;
+// The exhaustive choice among the exact encoded sizes (payload + 16 B
+// metadata) of every scheme, as the host exhaustive encoder gives them
+// (fls_host.cpp scheme_sizes), by the label rule of the learned selector:
+// argmin of size x (1 + kappa (decode cost - 1)) with the decode costs FOR 1,
+// DELTA 1.5, RLE 2, CONST 1, DICT 4.5, ties to the cheaper decode (FOR, CONST,
+// DELTA, RLE, DICT), in IEEE double with each product and sum rounded
+// separately (no fused multiply-add), as numpy computes it.
+__device__ uint32_t exhaustive_choice(double kappa, uint32_t range_bits, uint32_t delta_bits, uint32_t runs,
+                                      uint32_t distinct, bool constant) {
+	uint32_t size[FLS_N_SCHEMES];
+	size[FLS_SCHEME_FOR]   = 16u + 4u * payload_words(FLS_SCHEME_FOR, range_bits, 0u);
+	size[FLS_SCHEME_DELTA] = 16u + 4u * payload_words(FLS_SCHEME_DELTA, delta_bits, 0u);
+	size[FLS_SCHEME_RLE]   = 16u + 4u * payload_words(FLS_SCHEME_RLE, range_bits, runs);
+	size[FLS_SCHEME_CONST] = constant ? 16u : 0xffffffffu;
+	size[FLS_SCHEME_DICT]  = 16u + 4u * payload_words(FLS_SCHEME_DICT, range_bits, distinct);
+	const uint32_t order[FLS_N_SCHEMES] = {FLS_SCHEME_FOR, FLS_SCHEME_CONST, FLS_SCHEME_DELTA, FLS_SCHEME_RLE,
+	                                       FLS_SCHEME_DICT};
+	const double cost[FLS_N_SCHEMES] = {1.0, 1.5, 2.0, 1.0, 4.5}; // by scheme id
+	uint32_t     best = order[0];
+	double       best_score = 0.0;
+#pragma unroll
+	for (uint32_t i = 0; i < FLS_N_SCHEMES; ++i) {
+		const uint32_t sc = order[i];
+		if (size[sc] == 0xffffffffu) { continue; }
+		const double f     = __dadd_rn(1.0, __dmul_rn(kappa, cost[sc] - 1.0));
+		const double score = __dmul_rn(static_cast<double>(size[sc]), f);
+		if (i == 0 || score < best_score) {
+			best       = sc;
+			best_score = score;
+		}
 	}
-	if (s == FLS_SCHEME_CONST && mn != mx) { s = FLS_SCHEME_FOR; }
-	const uint32_t range = static_cast<uint32_t>(mx) - static_cast<uint32_t>(mn);
-	Plan           p {s, 0u, 0u, 0};
-	switch (s) {
+	return best;
+}
+
+// Scheme parameters of the staged vector (CONST on a non-constant vector
+// becomes FOR, as on the host).  LEARNED: `counts` are known, and a vector the
+// network is `unsure` of takes the exhaustive choice instead of `s`, which
+// receives it.
+template <bool LEARNED>
+__device__ __forceinline__ Plan plan_vector(const EncParams& P, uint64_t v, int32_t* sv, uint32_t lane, int32_t mn,
+                                            int32_t mx, uint32_t& s, const sel::Counts& counts, bool unsure) {
+	const uint32_t range_bits = bits_of(static_cast<uint32_t>(mx) - static_cast<uint32_t>(mn));
+	uint32_t       k[32], first = 0, before = 0, distinct = 0;
+	if (s == FLS_SCHEME_DICT || (LEARNED && unsure)) {
+		distinct = sort_distinct(sv, lane, mn, range_bits, k, first, before);
+	}
+	if constexpr (LEARNED) {
+		if (unsure) {
+			s = exhaustive_choice(P.kappa, range_bits, bits_of(counts.max_d), counts.runs, distinct, mn == mx);
+			if (s != FLS_SCHEME_DICT) { // the sort took the staged values' place
+				int32_t mn2, mx2;
+				__syncwarp();
+				sel::stage_vector(P.values, P.n, v, sv, lane, mn2, mx2);
+			}
+		}
+	}
+	Plan p {s, 0u, 0u, 0};
+	if (s == FLS_SCHEME_CONST && mn != mx) { p.scheme = FLS_SCHEME_FOR; }
+	switch (p.scheme) {
 	case FLS_SCHEME_CONST: p.base = mn; break;
 	case FLS_SCHEME_FOR:
-		p.bw = bits_of(range);
+		p.bw = range_bits;
 		if (P.round4 && p.bw) { p.bw = (p.bw + 3u) & ~3u; }
 		p.base = mn;
 		break;
 	case FLS_SCHEME_DELTA: {
-		const uint32_t c = dev::chunk_of_lane(lane);
-		uint32_t       mxd = 0;
-		int32_t        prev = val_at(sv, 32u * c);
-		for (uint32_t t = 1; t < 32; ++t) {
-			const int32_t cur = val_at(sv, 32u * c + t);
-			mxd               = max(mxd, static_cast<uint32_t>(cur) - static_cast<uint32_t>(prev));
-			prev              = cur;
+		uint32_t mxd = counts.max_d;
+		if constexpr (!LEARNED) {
+			int32_t prev = sv[33u * lane];
+			mxd          = 0;
+#pragma unroll 8
+			for (uint32_t t = 1; t < 32; ++t) {
+				const int32_t cur = sv[33u * lane + t];
+				mxd               = max(mxd, static_cast<uint32_t>(cur) - static_cast<uint32_t>(prev));
+				prev              = cur;
+			}
+			mxd = __reduce_max_sync(0xffffffffu, mxd);
 		}
-		p.bw = bits_of(__reduce_max_sync(0xffffffffu, mxd));
+		p.bw = bits_of(mxd);
 		break;
 	}
 	case FLS_SCHEME_RLE:
-		p.aux  = __reduce_add_sync(0xffffffffu, __popc(chunk_starts(sv, lane)));
-		p.bw   = bits_of(range);
+		p.aux  = LEARNED ? counts.runs : __reduce_add_sync(0xffffffffu, __popc(chunk_starts(sv, lane)));
+		p.bw   = range_bits;
 		p.base = mn;
 		break;
-	default: { // DICT: leaves the dictionary in u, and the codes in sv when the keys carry them
-		uint32_t k[32], first, before;
-		p.bw   = bits_of(range);
+	default: // DICT: the dictionary and the codes take the staged values' place
+		p.aux  = distinct;
+		p.bw   = range_bits;
 		p.base = mn;
-		p.aux  = sort_distinct(sv, u, lane, mn, p.bw, k, first, before);
-		write_dict(k, first, before, p.bw <= kKeyedBits, sv, u);
+		write_dict(k, first, before, p.bw <= kKeyedBits, sv);
 		break;
-	}
 	}
 	return p;
 }
 
-// ------------------------------------------------ learned selection
-
-struct SelParams {
-	const int32_t*      values;
-	uint64_t            n, n_vec;
-	const uint8_t*      mlp_best; // the network's pick per vector
-	const float*        conf;     // and its probability
-	float               threshold;
-	uint32_t            pad_;
-	double              kappa;
-	uint8_t*            schemes;  // the chosen scheme per vector
-	unsigned long long* n_fallback;
-};
-
-// The exhaustive choice for vectors the network is unsure of (confidence
-// below threshold), else the network's pick.  The exact encoded sizes of
-// every scheme (payload + 16 B metadata) are the host exhaustive encoder's
-// (fls_host.cpp scheme_sizes), the choice the label rule of the learned
-// selector: argmin of size x (1 + kappa (decode cost - 1)) with the decode
-// costs FOR 1, DELTA 1.5, RLE 2, CONST 1, DICT 4.5, ties to the cheaper
-// decode (FOR, CONST, DELTA, RLE, DICT), in IEEE double with each product and
-// sum rounded separately (no fused multiply-add), as numpy computes it.
-__global__ void __launch_bounds__(kEncWarps * 32) enc_select_kernel(const __grid_constant__ SelParams S) {
-	extern __shared__ __align__(16) int32_t esmem[];
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	int32_t*       sv   = esmem + warp * kEncWarpWords;
-	uint32_t*      u    = reinterpret_cast<uint32_t*>(sv + kValWords);
-	EncParams      P {};
-	P.values = S.values;
-	P.n      = S.n;
-	for (uint64_t v = static_cast<uint64_t>(blockIdx.x) * kEncWarps + warp; v < S.n_vec;
-	     v += static_cast<uint64_t>(gridDim.x) * kEncWarps) {
-		if (!(S.conf[v] < S.threshold)) {
-			if (lane == 0) { S.schemes[v] = S.mlp_best[v]; }
-			continue;
-		}
-		int32_t mn, mx;
-		stage_vector(P, v, sv, lane, mn, mx);
-		const uint32_t rbw = bits_of(static_cast<uint32_t>(mx) - static_cast<uint32_t>(mn));
-		uint32_t       mxd = 0;
-		{
-			const uint32_t c    = dev::chunk_of_lane(lane);
-			int32_t        prev = val_at(sv, 32u * c);
-			for (uint32_t t = 1; t < 32; ++t) {
-				const int32_t cur = val_at(sv, 32u * c + t);
-				mxd               = max(mxd, static_cast<uint32_t>(cur) - static_cast<uint32_t>(prev));
-				prev              = cur;
-			}
-		}
-		const uint32_t dbw    = bits_of(__reduce_max_sync(0xffffffffu, mxd));
-		const uint32_t n_runs = __reduce_add_sync(0xffffffffu, __popc(chunk_starts(sv, lane)));
-		uint32_t       k[32], first, before;
-		const uint32_t n_dist = sort_distinct(sv, u, lane, mn, rbw, k, first, before);
-		if (lane == 0) {
-			uint32_t size[FLS_N_SCHEMES];
-			size[FLS_SCHEME_FOR]   = 16u + 4u * payload_words(FLS_SCHEME_FOR, rbw, 0u);
-			size[FLS_SCHEME_DELTA] = 16u + 4u * payload_words(FLS_SCHEME_DELTA, dbw, 0u);
-			size[FLS_SCHEME_RLE]   = 16u + 4u * payload_words(FLS_SCHEME_RLE, rbw, n_runs);
-			size[FLS_SCHEME_CONST] = mn == mx ? 16u : 0xffffffffu;
-			size[FLS_SCHEME_DICT]  = 16u + 4u * payload_words(FLS_SCHEME_DICT, rbw, n_dist);
-			const uint32_t order[FLS_N_SCHEMES] = {FLS_SCHEME_FOR, FLS_SCHEME_CONST, FLS_SCHEME_DELTA, FLS_SCHEME_RLE,
-			                                       FLS_SCHEME_DICT};
-			const double cost[FLS_N_SCHEMES] = {1.0, 1.5, 2.0, 1.0, 4.5}; // by scheme id
-			uint32_t     best = order[0];
-			double       best_score = 0.0;
-			for (uint32_t i = 0; i < FLS_N_SCHEMES; ++i) {
-				const uint32_t sc = order[i];
-				if (size[sc] == 0xffffffffu) { continue; }
-				const double f     = __dadd_rn(1.0, __dmul_rn(S.kappa, cost[sc] - 1.0));
-				const double score = __dmul_rn(static_cast<double>(size[sc]), f);
-				if (i == 0 || score < best_score) {
-					best       = sc;
-					best_score = score;
-				}
-			}
-			S.schemes[v] = static_cast<uint8_t>(best);
-			atomicAdd(S.n_fallback, 1ull);
-		}
-		__syncwarp();
-	}
-}
-
 // Writes the planned vector's payload (staged in sv; DICT: planned) at `out`.
-__device__ __forceinline__ void write_vector(const EncParams& P, const Plan& p, const int32_t* sv, uint32_t* u,
-                                             uint32_t* out, uint32_t lane) {
+__device__ __forceinline__ void write_vector(const EncParams& P, uint64_t v, const Plan& p, int32_t* sv, uint32_t* out,
+                                             uint32_t lane) {
 	const uint32_t base  = static_cast<uint32_t>(p.base);
 	uint32_t       x[32] = {}, bw = 0, skip = 0; // rows to pack, their width, words before them
 	if (p.scheme == FLS_SCHEME_FOR) {
@@ -547,12 +496,16 @@ __device__ __forceinline__ void write_vector(const EncParams& P, const Plan& p, 
 			if (lane >= static_cast<uint32_t>(o)) { pre += y; }
 		}
 		pre -= cnt;
-		// run dictionary: the value at each start, in order
-		uint32_t ff = f, k = pre;
-		while (ff) {
-			const uint32_t t = __ffs(ff) - 1u;
-			ff &= ff - 1u;
-			u[k++] = static_cast<uint32_t>(sv[33u * lane + t]) - base;
+		// run dictionary: the value at each start, in order, in the place of
+		// the values
+		auto*    u = reinterpret_cast<uint32_t*>(sv);
+		uint32_t k = pre;
+#pragma unroll
+		for (uint32_t t = 0; t < 32; ++t) { x[t] = static_cast<uint32_t>(sv[33u * lane + t]) - base; }
+		__syncwarp();
+#pragma unroll
+		for (uint32_t t = 0; t < 32; ++t) {
+			if ((f >> t) & 1u) { u[k++] = x[t]; }
 		}
 		// transposed lane L holds chunk c(L): base = run index of its first
 		// value, then 1-bit deltas (a start) in rsum row order
@@ -570,16 +523,18 @@ __device__ __forceinline__ void write_vector(const EncParams& P, const Plan& p, 
 		__syncwarp();
 		pack_sequential(u, p.aux, p.bw, out + 48, lane);
 	} else if (p.scheme == FLS_SCHEME_DICT) {
-		const uint32_t n = p.aux;
-		bw               = bits_of(n - 1u);
+		const uint32_t  n = p.aux;
+		const uint32_t* u = dict_of(sv);
+		bw                = bits_of(n - 1u);
 		if (p.bw <= kKeyedBits) {
-			const uint16_t* codes = reinterpret_cast<const uint16_t*>(sv);
 #pragma unroll
-			for (uint32_t r = 0; r < 32; ++r) { x[r] = codes[code_pos(layout_index(P.layout, lane, r))]; }
-		} else {
+			for (uint32_t r = 0; r < 32; ++r) { x[r] = codes_of(sv)[code_pos(layout_index(P.layout, lane, r))]; }
+		} else { // the values once more, from the column
+			const uint64_t v0 = v * 1024u;
 #pragma unroll
 			for (uint32_t r = 0; r < 32; ++r) {
-				const uint32_t val = static_cast<uint32_t>(val_at(sv, layout_index(P.layout, lane, r))) - base;
+				const uint64_t i   = min(v0 + layout_index(P.layout, lane, r), P.n - 1u);
+				const uint32_t val = static_cast<uint32_t>(__ldg(P.values + i)) - base;
 				uint32_t       lo  = 0; // the value's position: it is there, so ten halvings find it
 #pragma unroll 1
 				for (uint32_t step = 512; step > 0; step >>= 1) {
@@ -593,59 +548,104 @@ __device__ __forceinline__ void write_vector(const EncParams& P, const Plan& p, 
 	pack_lane(x, bw, out + skip, lane);
 }
 
-// Bounded by the per-vector work of planning and packing (DICT: the sort) and,
-// for large columns, by how many vectors an SM has in flight: two 33-padded
-// buffers per warp let three CTAs (24 warps) share an SM.  Against separate
+// Bounded by the per-vector work of planning (DICT: the sort; LEARNED: the
+// statistics and the network, about 6 us of a round of 24 vectors per SM) and,
+// in columns of few rounds, by the round trip of a tile's offset, 2-4 us.
+// 1568 words per warp let three CTAs (24 warps) share an SM.  Against separate
 // plan, scan and write kernels, which read and sorted everything twice, whole
-// encoder calls took (us, before -> after): 6 M values DICT 437 -> 126,
-// 33.5 M values FOR 187 -> 168, DELTA 188 -> 165, RLE 186 -> 174, DICT 1918
-// -> 325; of each about 60 are the call's host side and its read-back.
+// encoder calls took (us, before -> after; about 60 of each are the call's
+// host side and its read-back): 6 M values DICT 437 -> 120, 33.5 M values FOR
+// 186 -> 120, DELTA 185 -> 118, RLE 185 -> 145, DICT 1920 -> 315.
+//
+// LEARNED: a warp first takes its vector's statistics and runs the network on
+// them (fls_selector.cuh), so the values are still read once and the column
+// takes one launch instead of eight (four columns of 8.4 M values: statistics
+// 20, network 21, choice 6, plan 18, scans 10, write 18-41 us each -> 40-50;
+// the whole call 576 -> 387 us).
+template <bool LEARNED>
 __global__ void __launch_bounds__(kEncWarps * 32, 3) enc_kernel(const __grid_constant__ EncParams P) {
 	extern __shared__ __align__(16) int32_t esmem[];
 	__shared__ uint32_t s_tile;
-	__shared__ uint64_t s_own[kEncWarps], s_before;
+	__shared__ uint32_t s_words[kEncWarps], s_mask[kEncWarps];
+	__shared__ uint64_t s_offset;
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	int32_t*       sv   = esmem + warp * kEncWarpWords;
-	uint32_t*      u    = reinterpret_cast<uint32_t*>(sv + kValWords);
+	float*         net  = reinterpret_cast<float*>(esmem + kEncWarps * kEncWarpWords); // LEARNED
+	uint32_t       fallbacks = 0; // of this warp's vectors
+	if constexpr (LEARNED) { sel::WarpNet::load(P.params, net); }
 	for (;;) {
+		// taken only now: a tile taken ahead of its work would hold up every
+		// tile after it
 		if (threadIdx.x == 0) { s_tile = atomicAdd(P.counter, 1u); }
 		__syncthreads();
-		const uint64_t tile = s_tile;
+		if (s_tile == 0u) { // the first ticket: this CTA adds up the tiles
+			if (warp == 0) { scan_tiles(P.reports, P.offsets, P.n_tiles, P.info, P.err, lane); }
+			break;
+		}
+		const uint64_t tile = s_tile - 1u;
 		if (tile >= P.n_tiles) { break; }
 		const uint64_t v    = tile * kEncWarps + warp;
 		const bool     live = v < P.n_vec;
 		Plan           p {};
 		uint32_t       words = 0;
-		if (live) {
-			int32_t mn, mx;
-			stage_vector(P, v, sv, lane, mn, mx);
-			p     = plan_vector(P, v, sv, u, lane, mn, mx);
-			words = payload_words(p.scheme, p.bw, p.aux);
+		int32_t        mn = 0, mx = 0;
+		sel::Counts    counts {};
+		uint32_t       scheme = 0;
+		bool           unsure = false;
+		if (live) { sel::stage_vector(P.values, P.n, v, sv, lane, mn, mx); }
+		// the vector this warp is likely to take next: from memory to L2
+		const uint64_t ahead = v + static_cast<uint64_t>(gridDim.x) * kEncWarps;
+		if ((ahead + 1u) * 1024u <= P.n) {
+			asm volatile("prefetch.global.L2 [%0];" ::"l"(P.values + ahead * 1024u + 32u * lane));
 		}
-		if (lane == 0) { s_own[warp] = live ? tile_state(words, words, 1u << p.scheme) : 0ull; }
+		if constexpr (LEARNED) {
+			if (live) {
+				const float f = sel::vector_features(sv, mn, mx, reinterpret_cast<uint8_t*>(sv + sel::kPadded), lane, counts);
+				float       z[sel::kOut], top;
+				sel::WarpNet::forward(net, reinterpret_cast<float*>(sv + kNetWords), f, lane, z);
+				sel::softmax5(z);
+				scheme = static_cast<uint32_t>(sel::top_of(z, top));
+				unsure = top < P.threshold;
+				__syncwarp(); // the activations are read before the warp's words serve something else
+			}
+		} else if (live) {
+			scheme = P.schemes ? P.schemes[v] : P.scheme;
+			if (scheme >= FLS_N_SCHEMES) {
+				if (lane == 0) { atomicOr(P.err, kErrBadMeta); }
+				scheme = FLS_SCHEME_FOR;
+			}
+		}
+		if (live) {
+			p     = plan_vector<LEARNED>(P, v, sv, lane, mn, mx, scheme, counts, unsure);
+			words = payload_words(p.scheme, p.bw, p.aux);
+			if (LEARNED && P.picks && lane == 0) { P.picks[v] = static_cast<uint8_t>(scheme); }
+		}
+		fallbacks += unsure ? 1u : 0u;
+		if (lane == 0) {
+			s_words[warp] = words;
+			s_mask[warp]  = live ? 1u << p.scheme : 0u;
+		}
 		__syncthreads();
 		if (warp == 0) {
-			uint64_t own = 0;
-#pragma unroll
-			for (uint32_t w = 0; w < kEncWarps; ++w) { own = tile_join(own, s_own[w]); }
-			const uint64_t before = tile_lookback(P.tiles, tile, own, lane);
+			const uint32_t w = lane < kEncWarps ? s_words[lane] : 0u, m = lane < kEncWarps ? s_mask[lane] : 0u;
+			const uint64_t own = tile_report(__reduce_add_sync(0xffffffffu, w), __reduce_max_sync(0xffffffffu, w),
+			                                 __reduce_or_sync(0xffffffffu, m));
 			if (lane == 0) {
-				s_before = before;
-				if (before == kTileLost) {
+				tile_store(P.reports + tile, own);
+				uint64_t got = 0;
+				for (uint32_t poll = 0; poll < kPollLimit && got == 0ull; ++poll) { got = tile_load(P.offsets + tile); }
+				if (got == 0ull) {
 					atomicOr(P.err, kErrTimeout);
-				} else if (tile + 1u == P.n_tiles) {
-					const uint64_t all = tile_join(before, own);
-					P.info[0]          = all & kTileSum;
-					P.info[1]          = tile_max(all);
-					P.info[2]          = tile_mask(all);
+					got = kTileLost;
 				}
+				s_offset = got;
 			}
 		}
 		__syncthreads();
-		const uint64_t before = s_before;
+		const uint64_t before = s_offset;
 		if (live && before != kTileLost) {
-			uint64_t offset = before & kTileSum;
-			for (uint32_t w = 0; w < warp; ++w) { offset += s_own[w] & kTileSum; }
+			uint64_t offset = before & ~kTileMark;
+			for (uint32_t w = 0; w < warp; ++w) { offset += s_words[w]; }
 			if (lane == 0) {
 				fls_vec_meta m;
 				m.offset  = offset;
@@ -655,10 +655,80 @@ __global__ void __launch_bounds__(kEncWarps * 32, 3) enc_kernel(const __grid_con
 				m.aux     = static_cast<uint16_t>(p.aux);
 				P.meta[v] = m;
 			}
-			write_vector(P, p, sv, u, P.out + offset, lane);
+			write_vector(P, v, p, sv, P.out + offset, lane);
 		}
-		__syncthreads(); // s_own and the staged vector are read before the next tile's
+		__syncthreads(); // s_words is read before the next tile's
 	}
+	if constexpr (LEARNED) {
+		// The last CTA to get here reports the fallbacks of all.
+		if (lane == 0 && fallbacks) { atomicAdd(P.n_fallback, static_cast<unsigned long long>(fallbacks)); }
+		__threadfence();
+		__syncthreads();
+		if (threadIdx.x == 0 && atomicAdd(P.counter + 1, 1u) + 1u == gridDim.x) {
+			__threadfence();
+			P.info[3] = atomicAdd(P.n_fallback, 0ull);
+		}
+	}
+}
+
+uint64_t workspace_bytes_of(uint64_t n) {
+	const uint64_t n_vec = (n + 1023u) / 1024u, n_tiles = (n_vec + kEncWarps - 1) / kEncWarps;
+	return 16u * n_tiles + 256u; // the counters, the tiles' reports and offsets, after alignment
+}
+
+// Checks the arguments both encoders share, fills in the rest of P and
+// launches the kernel: one memset of the tiles' states, one launch.
+template <bool LEARNED>
+fls_status encode_launch(EncParams& P, uint64_t out_capacity_words, void* d_workspace, uint64_t workspace_bytes,
+                         cudaStream_t st, const std::string& who) {
+	if (!P.values || !P.out || !P.meta || !P.info || !d_workspace || P.n == 0) {
+		return set_error(FLS_ERR_INVALID_ARG, who + ": null pointer or n == 0");
+	}
+	if (fls_status s = check_n_values(P.n, who.c_str()); s != FLS_OK) { return s; }
+	if (P.layout > FLS_LAYOUT_TRANSPOSED) { return set_error(FLS_ERR_INVALID_ARG, who + ": bad layout"); }
+	if ((reinterpret_cast<uintptr_t>(P.out) | reinterpret_cast<uintptr_t>(P.meta)) & 15u) {
+		return set_error(FLS_ERR_ALIGNMENT, who + ": output and metadata must be 16-byte aligned");
+	}
+	P.n_vec = (P.n + 1023u) / 1024u;
+	if (out_capacity_words < P.n_vec * kMaxVecWords) {
+		return set_error(FLS_ERR_CAPACITY, who + ": output smaller than fls_encode_bound_words(n)");
+	}
+	if (workspace_bytes < workspace_bytes_of(P.n)) {
+		return set_error(FLS_ERR_CAPACITY, who + ": workspace smaller than " +
+		                                       (LEARNED ? "fls_encode_learned_workspace_bytes(n)" : "fls_encode_gpu_workspace_bytes(n)"));
+	}
+	DeviceInfo di;
+	fls_status s = device_info(di);
+	if (s != FLS_OK) { return s; }
+	char* ws     = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(d_workspace) + 15u) & ~uintptr_t {15u});
+	P.n_tiles    = (P.n_vec + kEncWarps - 1) / kEncWarps;
+	P.counter    = reinterpret_cast<uint32_t*>(ws);
+	P.n_fallback = reinterpret_cast<unsigned long long*>(ws + 8);
+	P.reports    = reinterpret_cast<uint64_t*>(ws + 16);
+	P.offsets    = P.reports + P.n_tiles;
+	P.err        = device_error_word(st);
+	const size_t smem = 4u * (kEncWarps * kEncWarpWords + (LEARNED ? sel::WarpNet::kFloats : 0u));
+	{
+		static std::mutex mu;
+		static uint64_t   configured = 0;
+		int               dev        = 0;
+		cudaGetDevice(&dev);
+		std::lock_guard<std::mutex> lk(mu);
+		if (dev >= 64 || !(configured & (1ull << dev))) {
+			if ((s = cuda_check(cudaFuncSetAttribute(enc_kernel<LEARNED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+			                                         static_cast<int>(smem)),
+			                    "cudaFuncSetAttribute")) != FLS_OK) {
+				return s;
+			}
+			if (dev < 64) { configured |= 1ull << dev; }
+		}
+	}
+	if ((s = cuda_check(cudaMemsetAsync(ws, 0, 16u + 16u * P.n_tiles, st), "cudaMemsetAsync")) != FLS_OK) { return s; }
+	const uint32_t grid =
+	    static_cast<uint32_t>(std::min<uint64_t>(P.n_tiles + 1u, static_cast<uint64_t>(di.sms) * 3u));
+	enc_kernel<LEARNED><<<grid, kEncWarps * 32, smem, st>>>(P);
+	count_launch();
+	return cuda_check(cudaGetLastError(), "enc_kernel launch");
 }
 
 } // namespace
@@ -668,145 +738,51 @@ using namespace fls;
 
 extern "C" {
 
-uint64_t fls_encode_gpu_workspace_bytes(uint64_t n) {
-	const uint64_t n_vec = (n + 1023u) / 1024u, n_tiles = (n_vec + kEncWarps - 1) / kEncWarps;
-	return 8u * n_tiles + 256u; // the counter and the tiles' states, after alignment
-}
+uint64_t fls_encode_gpu_workspace_bytes(uint64_t n) { return workspace_bytes_of(n); }
 
 fls_status fls_encode_column_gpu(const int32_t* d_values, uint64_t n, const uint8_t* d_schemes, uint32_t scheme,
                                  uint32_t layout, int round4, uint32_t* d_out, uint64_t out_capacity_words,
                                  fls_vec_meta* d_meta, uint64_t* d_info, void* d_workspace, uint64_t workspace_bytes,
                                  fls_stream_t stream) {
-	if (!d_values || !d_out || !d_meta || !d_info || !d_workspace || n == 0) {
-		return set_error(FLS_ERR_INVALID_ARG, "fls_encode_column_gpu: null pointer or n == 0");
-	}
-	if (fls_status s = check_n_values(n, "fls_encode_column_gpu"); s != FLS_OK) { return s; }
 	if (!d_schemes && scheme >= FLS_N_SCHEMES) { return set_error(FLS_ERR_INVALID_ARG, "fls_encode_column_gpu: bad scheme"); }
-	if (layout > FLS_LAYOUT_TRANSPOSED) { return set_error(FLS_ERR_INVALID_ARG, "fls_encode_column_gpu: bad layout"); }
-	if ((reinterpret_cast<uintptr_t>(d_out) | reinterpret_cast<uintptr_t>(d_meta)) & 15u) {
-		return set_error(FLS_ERR_ALIGNMENT, "fls_encode_column_gpu: output and metadata must be 16-byte aligned");
-	}
-	const uint64_t n_vec = (n + 1023u) / 1024u;
-	if (out_capacity_words < n_vec * kMaxVecWords) {
-		return set_error(FLS_ERR_CAPACITY, "fls_encode_column_gpu: output smaller than fls_encode_bound_words(n)");
-	}
-	if (workspace_bytes < fls_encode_gpu_workspace_bytes(n)) {
-		return set_error(FLS_ERR_CAPACITY, "fls_encode_column_gpu: workspace smaller than fls_encode_gpu_workspace_bytes(n)");
-	}
-	DeviceInfo di;
-	fls_status s = device_info(di);
-	if (s != FLS_OK) { return s; }
-	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-	EncParams    P {};
+	EncParams P {};
 	P.values  = d_values;
 	P.n       = n;
-	P.n_vec   = n_vec;
 	P.schemes = d_schemes;
 	P.scheme  = scheme;
 	P.layout  = layout;
 	P.round4  = round4 ? 1u : 0u;
 	P.out     = d_out;
 	P.meta    = d_meta;
-	char* ws  = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(d_workspace) + 15u) & ~uintptr_t {15u});
-	P.n_tiles = (n_vec + kEncWarps - 1) / kEncWarps;
-	P.counter = reinterpret_cast<uint32_t*>(ws);
-	P.tiles   = reinterpret_cast<uint64_t*>(ws + 16);
 	P.info    = d_info;
-	P.err     = device_error_word(st);
-	const size_t smem = 4u * kEncWarps * kEncWarpWords;
-	{
-		static std::mutex mu;
-		static uint64_t   configured = 0;
-		int               dev        = 0;
-		cudaGetDevice(&dev);
-		std::lock_guard<std::mutex> lk(mu);
-		if (dev >= 64 || !(configured & (1ull << dev))) {
-			if ((s = cuda_check(cudaFuncSetAttribute(enc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                                         static_cast<int>(smem)),
-			                    "cudaFuncSetAttribute")) != FLS_OK) {
-				return s;
-			}
-			if (dev < 64) { configured |= 1ull << dev; }
-		}
-	}
-	if ((s = cuda_check(cudaMemsetAsync(ws, 0, 16u + 8u * P.n_tiles, st), "cudaMemsetAsync")) != FLS_OK) { return s; }
-	const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(P.n_tiles, static_cast<uint64_t>(di.sms) * 8u));
-	enc_kernel<<<grid, kEncWarps * 32, smem, st>>>(P);
-	count_launch();
-	return cuda_check(cudaGetLastError(), "enc_kernel launch");
+	return encode_launch<false>(P, out_capacity_words, d_workspace, workspace_bytes,
+	                            reinterpret_cast<cudaStream_t>(stream), "fls_encode_column_gpu");
 }
 
-uint64_t fls_encode_learned_workspace_bytes(uint64_t n) {
-	const uint64_t n_vec = (n + 1023u) / 1024u;
-	auto           a256  = [](uint64_t b) { return (b + 255u) & ~uint64_t {255u}; };
-	return a256(64u * n_vec) + a256(4u * n_vec) + 2u * a256(n_vec) + fls_encode_gpu_workspace_bytes(n);
-}
+uint64_t fls_encode_learned_workspace_bytes(uint64_t n) { return workspace_bytes_of(n); }
 
 fls_status fls_encode_learned_gpu(const int32_t* d_values, uint64_t n, const float* d_params, float threshold,
                                   double kappa, uint32_t layout, uint32_t* d_out, uint64_t out_capacity_words,
                                   fls_vec_meta* d_meta, uint64_t* d_info, uint8_t* d_schemes, void* d_workspace,
                                   uint64_t workspace_bytes, fls_stream_t stream) {
-	if (!d_values || !d_params || !d_info || !d_workspace || n == 0) {
-		return set_error(FLS_ERR_INVALID_ARG, "fls_encode_learned_gpu: null pointer or n == 0");
-	}
-	if (fls_status s = check_n_values(n, "fls_encode_learned_gpu"); s != FLS_OK) { return s; }
+	if (!d_params) { return set_error(FLS_ERR_INVALID_ARG, "fls_encode_learned_gpu: null pointer or n == 0"); }
 	if (!(kappa >= 0.0)) { return set_error(FLS_ERR_INVALID_ARG, "fls_encode_learned_gpu: kappa must be >= 0"); }
-	if (workspace_bytes < fls_encode_learned_workspace_bytes(n) || (reinterpret_cast<uintptr_t>(d_workspace) & 255u)) {
-		return set_error(FLS_ERR_CAPACITY,
-		                 "fls_encode_learned_gpu: workspace smaller than fls_encode_learned_workspace_bytes(n) "
-		                 "or not 256-byte aligned");
+	if (reinterpret_cast<uintptr_t>(d_workspace) & 255u) {
+		return set_error(FLS_ERR_CAPACITY, "fls_encode_learned_gpu: workspace not 256-byte aligned");
 	}
-	const uint64_t n_vec = (n + 1023u) / 1024u;
-	auto           a256  = [](uint64_t b) { return (b + 255u) & ~uint64_t {255u}; };
-	char*          w     = static_cast<char*>(d_workspace);
-	float*         stats = reinterpret_cast<float*>(w);
-	float*         conf  = reinterpret_cast<float*>(w + a256(64u * n_vec));
-	uint8_t*       best  = reinterpret_cast<uint8_t*>(w + a256(64u * n_vec) + a256(4u * n_vec));
-	uint8_t*       own   = best + a256(n_vec);
-	void*          enc   = own + a256(n_vec);
-	uint8_t*       pick  = d_schemes ? d_schemes : own;
-	cudaStream_t   st    = reinterpret_cast<cudaStream_t>(stream);
-	DeviceInfo     di;
-	fls_status     s = device_info(di);
-	if (s != FLS_OK) { return s; }
-	if ((s = fls_vector_stats_gpu(d_values, n, stats, stream)) != FLS_OK) { return s; }
-	if ((s = fls_mlp_infer(d_params, stats, n_vec, nullptr, best, conf, stream)) != FLS_OK) { return s; }
-	const size_t smem = 4u * kEncWarps * kEncWarpWords;
-	{
-		static std::mutex mu;
-		static uint64_t   configured = 0;
-		int               dev        = 0;
-		cudaGetDevice(&dev);
-		std::lock_guard<std::mutex> lk(mu);
-		if (dev >= 64 || !(configured & (1ull << dev))) {
-			if ((s = cuda_check(cudaFuncSetAttribute(enc_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			                                         static_cast<int>(smem)),
-			                    "cudaFuncSetAttribute")) != FLS_OK) {
-				return s;
-			}
-			if (dev < 64) { configured |= 1ull << dev; }
-		}
-	}
-	if ((s = cuda_check(cudaMemsetAsync(d_info + 3, 0, sizeof(uint64_t), st), "cudaMemsetAsync")) != FLS_OK) {
-		return s;
-	}
-	SelParams S {};
-	S.values     = d_values;
-	S.n          = n;
-	S.n_vec      = n_vec;
-	S.mlp_best   = best;
-	S.conf       = conf;
-	S.threshold  = threshold;
-	S.kappa      = kappa;
-	S.schemes    = pick;
-	S.n_fallback = reinterpret_cast<unsigned long long*>(d_info + 3);
-	const uint32_t grid = static_cast<uint32_t>(
-	    std::min<uint64_t>((n_vec + kEncWarps - 1) / kEncWarps, static_cast<uint64_t>(di.sms) * 8u));
-	enc_select_kernel<<<grid, kEncWarps * 32, smem, st>>>(S);
-	count_launch(1);
-	if ((s = cuda_check(cudaGetLastError(), "enc_select_kernel launch")) != FLS_OK) { return s; }
-	return fls_encode_column_gpu(d_values, n, pick, 0u, layout, 0, d_out, out_capacity_words, d_meta, d_info, enc,
-	                             fls_encode_gpu_workspace_bytes(n), stream);
+	EncParams P {};
+	P.values    = d_values;
+	P.n         = n;
+	P.layout    = layout;
+	P.out       = d_out;
+	P.meta      = d_meta;
+	P.info      = d_info;
+	P.params    = d_params;
+	P.threshold = threshold;
+	P.kappa     = kappa;
+	P.picks     = d_schemes;
+	return encode_launch<true>(P, out_capacity_words, d_workspace, workspace_bytes,
+	                           reinterpret_cast<cudaStream_t>(stream), "fls_encode_learned_gpu");
 }
 
 } // extern "C"

@@ -5,146 +5,32 @@
 // bit width is always recomputed exactly by the encoder, so any pick is
 // lossless.  (No reference counterpart: the reference chooses encodings by hand
 // per column, ssb_utils.h:37-83.)
-//
-// Parameter layout (FLS_MLP_N_PARAMS floats): W1[64][16], b1[64], W2[64][64],
-// b2[64], W3[5][64], b3[5]; ReLU after layers 1 and 2, softmax cross-entropy.
 #include <cuda_runtime.h>
 
 #include <mutex>
 #include <vector>
 
-#include "fls_pipeline.cuh"
+#include "fls_selector.cuh"
 
 namespace fls {
 namespace {
 
-constexpr int kIn = FLS_MLP_IN, kH = FLS_MLP_HIDDEN, kOut = FLS_MLP_OUT;
-constexpr int kW1 = 0, kB1 = kW1 + kH * kIn, kW2 = kB1 + kH, kB2 = kW2 + kH * kH, kW3 = kB2 + kH,
-              kB3 = kW3 + kOut * kH, kNP = kB3 + kOut;
-static_assert(kNP == FLS_MLP_N_PARAMS, "parameter layout");
-
-__device__ __forceinline__ uint32_t bits32(uint32_t v) { return 32u - static_cast<uint32_t>(__clz(v)); }
+using namespace sel;
 
 // ------------------------------------------------------ vector statistics
-
-// Value j of a vector staged with one pad word per 32 values: lane L's
-// chunk (values 32L..32L+31) is then read without bank conflicts.
-__device__ __forceinline__ uint32_t pad33(uint32_t j) { return j + (j >> 5); }
 
 // One warp per vector; exactly the features of vector_stats() (fls_host.cpp).
 __global__ void __launch_bounds__(256) stats_kernel(const int32_t* __restrict__ values, uint64_t n, uint64_t n_vec,
                                                     float* __restrict__ out) {
-	__shared__ int32_t  vbuf[8][1056];
-	__shared__ uint32_t bmap[8][32];
+	__shared__ int32_t                vbuf[8][kPadded];
+	__shared__ __align__(16) uint8_t  buckets[8][kBuckets];
 	const uint32_t lane = threadIdx.x & 31u, wi = threadIdx.x >> 5;
 	const uint64_t warps = static_cast<uint64_t>(gridDim.x) * 8u;
-	int32_t*       v     = vbuf[wi];
-	uint32_t*      bm    = bmap[wi];
 	for (uint64_t vec = static_cast<uint64_t>(blockIdx.x) * 8u + wi; vec < n_vec; vec += warps) {
-		const uint64_t start = vec * 1024u;
-		const uint32_t cnt   = static_cast<uint32_t>(n - start < 1024u ? n - start : 1024u);
-		int32_t        mn = INT32_MAX, mx = INT32_MIN;
-		if (cnt == 1024u && (reinterpret_cast<uintptr_t>(values) & 15u) == 0) { // warp-uniform
-			// eight 16-byte loads per lane (values 128 k + 4 lane .. + 3), all
-			// in flight, then stored 33-padded (conflict-free: (j + j / 32)
-			// mod 32 differs across lanes)
-			int4 q[8];
-#pragma unroll
-			for (uint32_t k = 0; k < 8; ++k) { q[k] = __ldg(reinterpret_cast<const int4*>(values + start) + 32u * k + lane); }
-#pragma unroll
-			for (uint32_t k = 0; k < 8; ++k) {
-				const uint32_t j    = 128u * k + 4u * lane;
-				const int32_t  e[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
-#pragma unroll
-				for (uint32_t t = 0; t < 4; ++t) {
-					v[pad33(j + t)] = e[t];
-					mn              = min(mn, e[t]);
-					mx              = max(mx, e[t]);
-				}
-			}
-		} else {
-			for (uint32_t j = lane; j < 1024u; j += 32u) {
-				// a partial last vector is padded with its last value (as the encoder does)
-				const int32_t x = values[start + min(j, cnt - 1u)];
-				v[pad33(j)]     = x;
-				mn              = min(mn, x);
-				mx              = max(mx, x);
-			}
-		}
-		bm[lane] = 0u;
-		__syncwarp();
-		mn = __reduce_min_sync(0xffffffffu, mn);
-		mx = __reduce_max_sync(0xffffffffu, mx);
-		const uint32_t rbw = bits32(static_cast<uint32_t>(mx) - static_cast<uint32_t>(mn));
-		const int32_t* c   = v + 33u * lane; // this lane's chunk: values 32 lane .. 32 lane + 31
-		// u <= tm_h (tm_q): the value lies in the lower half (sixteenth) of the
-		// range's bit width; every value counts when the width is 0 (<= 4)
-		const uint32_t tm_h = rbw == 0 ? 0xffffffffu : (1u << (rbw / 2)) - 1u;
-		const uint32_t tm_q = rbw <= 4 ? 0xffffffffu : (1u << (rbw - 4)) - 1u;
-		const int32_t  c0   = c[0];
-		// the value before the chunk; the vector's first value is compared
-		// with itself (an equal pair, corrected below)
-		const int32_t  pb   = lane ? v[pad33(32u * lane - 1u)] : c0;
-		int32_t        p    = pb;
-		uint32_t       max_d = 0, up = 0, eqs = 0, lh = 0, lq = 0;
-		unsigned long long sabs = 0;
-		bool               same = true;
-#pragma unroll 8
-		for (uint32_t s = 0; s < 32; ++s) {
-			const int32_t  x = c[s];
-			const uint32_t u = static_cast<uint32_t>(x) - static_cast<uint32_t>(mn);
-			lh += u <= tm_h ? 1u : 0u;
-			lq += u <= tm_q ? 1u : 0u;
-			const uint32_t h = (static_cast<uint32_t>(x) * 0x9e3779b1u) >> 22;
-			atomicOr(&bm[h >> 5], 1u << (h & 31u));
-			same = same && x == c0;
-			sabs += static_cast<uint32_t>(max(x, p)) - static_cast<uint32_t>(min(x, p));
-			up += x > p ? 1u : 0u;
-			eqs += x == p ? 1u : 0u;
-			if (s != 0) { max_d = max(max_d, static_cast<uint32_t>(x) - static_cast<uint32_t>(p)); }
-			p = x;
-		}
-		// deltas of the lane: 32 (31 for lane 0, whose first value has no
-		// predecessor); runs (rle.hpp): a change of value, or every 256 values
-		// (the chunks of lanes 0, 8, 16, 24 open one whether or not the value
-		// changes, lane 0's first value included)
-		uint32_t       eq   = eqs - (lane == 0 ? 1u : 0u);
-		uint32_t       down = 32u - up - eqs;
-		uint32_t       runs = 32u - eqs + (((lane & 7u) == 0 && c0 == pb) ? 1u : 0u);
-		__syncwarp();
-		const uint32_t occ = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(__popc(bm[lane])));
-		max_d              = __reduce_max_sync(0xffffffffu, max_d);
-		runs               = __reduce_add_sync(0xffffffffu, runs);
-		up                 = __reduce_add_sync(0xffffffffu, up);
-		down               = __reduce_add_sync(0xffffffffu, down);
-		eq                 = __reduce_add_sync(0xffffffffu, eq);
-		lh                 = __reduce_add_sync(0xffffffffu, lh);
-		lq                 = __reduce_add_sync(0xffffffffu, lq);
-		const uint32_t cc  = static_cast<uint32_t>(__popc(__ballot_sync(0xffffffffu, same)));
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) { sabs += __shfl_xor_sync(0xffffffffu, sabs, o); }
-		const unsigned long long mean_d = sabs >> 10;
-		const uint32_t amin = mn < 0 ? static_cast<uint32_t>(-static_cast<long long>(mn)) : static_cast<uint32_t>(mn);
-		float f = 0.0f;
-		switch (lane) {
-		case 0: f = static_cast<float>(rbw) / 32.0f; break;
-		case 1: f = static_cast<float>(bits32(max_d)) / 32.0f; break;
-		case 2: f = static_cast<float>(runs) / 1024.0f; break;
-		case 3: f = static_cast<float>(up) / 1024.0f; break;
-		case 4: f = static_cast<float>(down) / 1024.0f; break;
-		case 5: f = static_cast<float>(eq) / 1024.0f; break;
-		case 6: f = static_cast<float>(occ) / 1024.0f; break;
-		case 7: f = static_cast<float>(bits32(occ)) / 16.0f; break;
-		case 8: f = static_cast<float>(bits32(static_cast<uint32_t>(min(mean_d, 0xffffffffull)))) / 32.0f; break;
-		case 9: f = static_cast<float>(lh) / 1024.0f; break;
-		case 10: f = static_cast<float>(lq) / 1024.0f; break;
-		case 11: f = static_cast<float>(bits32(amin)) / 32.0f; break;
-		case 12: f = mn == mx ? 1.0f : 0.0f; break;
-		case 13: f = static_cast<float>(bits32(runs)) / 16.0f; break;
-		case 14: f = static_cast<float>(cc) / 32.0f; break;
-		case 15: f = 1.0f; break;
-		default: break;
-		}
+		int32_t mn, mx;
+		stage_vector(values, n, vec, vbuf[wi], lane, mn, mx);
+		Counts      counts;
+		const float f = vector_features(vbuf[wi], mn, mx, buckets[wi], lane, counts);
 		if (lane < 16) { out[vec * 16u + lane] = f; }
 		__syncwarp();
 	}
@@ -234,21 +120,6 @@ __device__ __forceinline__ void forward_one(const float* __restrict__ P, const f
 	}
 }
 
-__device__ __forceinline__ void softmax5(float (&z)[kOut]) {
-	float m = z[0];
-#pragma unroll
-	for (int k = 1; k < kOut; ++k) { m = fmaxf(m, z[k]); }
-	float s = 0.0f;
-#pragma unroll
-	for (int k = 0; k < kOut; ++k) {
-		z[k] = expf(z[k] - m);
-		s += z[k];
-	}
-	const float inv = 1.0f / s;
-#pragma unroll
-	for (int k = 0; k < kOut; ++k) { z[k] *= inv; }
-}
-
 __global__ void __launch_bounds__(256, 2) mlp_infer_kernel(const float* __restrict__ params, const float* __restrict__ x,
                                                         uint64_t n, float* __restrict__ probs, uint8_t* __restrict__ best,
                                                         float* __restrict__ conf) {
@@ -262,15 +133,8 @@ __global__ void __launch_bounds__(256, 2) mlp_infer_kernel(const float* __restri
 		float h1[kH], z[kOut];
 		forward_one(P, x + i * kIn, h1, z, nullptr);
 		softmax5(z);
-		int   arg = 0;
-		float top = z[0];
-#pragma unroll
-		for (int k = 1; k < kOut; ++k) {
-			if (z[k] > top) {
-				top = z[k];
-				arg = k;
-			}
-		}
+		float     top;
+		const int arg = top_of(z, top);
 		if (probs) {
 #pragma unroll
 			for (int k = 0; k < kOut; ++k) { probs[i * kOut + k] = z[k]; }

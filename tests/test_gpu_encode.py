@@ -115,10 +115,11 @@ def test_gpu_encoder_dictionary_ranges(cuda, bits, n_distinct):
         _compare(vals, 4, layout)
 
 
-@pytest.mark.parametrize("n_vec", [7, 8, 9, 8 * 32 + 1, 8 * 128, 8 * 128 + 8, 8 * 129 + 3, 8 * 1500 + 5])
+@pytest.mark.parametrize("n_vec", [7, 8, 9, 8 * 32 + 1, 8 * 128, 8 * 256, 8 * 257 + 3, 8 * 1500 + 5])
 def test_gpu_encoder_offsets_over_many_tiles(cuda, n_vec):
-    """Offsets, total, largest vector and scheme mask around the look-back's
-    window (128 tiles of 8 vectors) and past the resident CTAs."""
+    """Offsets, total, largest vector and scheme mask around the tiles of 8
+    vectors, the scan's groups of 32 and rounds of 256 tiles, and past the
+    resident CTAs."""
     g = np.random.default_rng(n_vec)
     vals = (g.integers(0, 1 << 31, (n_vec, 1024)) >> g.integers(0, 31, (n_vec, 1))).astype(np.int32).reshape(-1)[:-11]
     schemes = np.where(g.integers(0, 50, n_vec) == 0, g.integers(0, 5, n_vec), 0).astype(np.uint8)
