@@ -39,6 +39,8 @@ struct fls_batch {
 	uint32_t                     slot_words = 0;
 	uint32_t                     has_dict   = 0;
 	bool                         any_pair   = false; // some query aggregates another column than it filters
+	uint32_t                     longest    = 0;     // most vectors of an item
+	uint64_t                     vectors    = 0;     // of all items
 	void*                        ws         = nullptr; // device workspace after upload
 	uint64_t                     ws_bytes   = 0;
 };
@@ -46,15 +48,17 @@ struct fls_batch {
 namespace fls {
 namespace {
 
-constexpr uint32_t kBatchStages = 3;
+constexpr uint32_t kBatchStages   = 3;
+constexpr uint32_t kPiecesPerWarp = 4;
 
 struct BatchParams {
 	const DevCol*          cols;
 	const fls_batch_query* queries;
 	const BatchGroup*      groups;
 	const uint4*           items;
-	uint32_t               n_items;
-	uint32_t*              counter;
+	uint64_t               n_pieces; // pieces_per_item * items
+	uint32_t               pieces_per_item, piece; // pieces of at most `piece` vectors
+	unsigned long long*    counter;
 	long long*             results; // 2 per query: sum, count
 	uint32_t               slot_words;
 	uint32_t               n_slots; // staged columns per stage: 1 (filter = aggregate everywhere) or 2
@@ -118,12 +122,18 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) batch_kernel(const __grid_c
 	__syncwarp();
 	const uint64_t pol   = dev::l2_evict_first_policy();
 	uint32_t       phase = 0, st = 0; // running stage / phase across items
+	// the piece after the current one is taken while that one is worked on
+	unsigned long long next = 0;
+	if (lane == 0) { next = atomicAdd(P.counter, 1ull); }
 	for (;;) {
-		uint32_t item = 0;
-		if (lane == 0) { item = atomicAdd(P.counter, 1u); }
-		item = __shfl_sync(0xffffffffu, item, 0);
-		if (item >= P.n_items) { break; }
-		const uint4       it = P.items[item];
+		const uint64_t piece = __shfl_sync(0xffffffffu, next, 0);
+		if (piece >= P.n_pieces) { break; }
+		if (lane == 0) { next = atomicAdd(P.counter, 1ull); }
+		const uint64_t    item = piece / P.pieces_per_item;
+		uint4             it   = P.items[item];
+		it.y += static_cast<uint32_t>(piece - item * P.pieces_per_item) * P.piece;
+		if (it.y >= it.z) { continue; } // a shorter item has fewer pieces
+		it.z = min(it.z, it.y + P.piece);
 		const BatchGroup  gr = P.groups[it.x];
 		const DevCol&     cf = P.cols[gr.col];
 		const DevCol&     ca = P.cols[gr.agg_col];
@@ -262,12 +272,12 @@ struct WsLayout {
 
 // Shared by fls_batch_run and its static-scratch variant.
 fls_status batch_launch(const fls_batch* b, const DevCol* cols, const fls_batch_query* queries,
-                        const BatchGroup* groups, const uint4* items, uint32_t* counter, int64_t* d_results,
+                        const BatchGroup* groups, const uint4* items, unsigned long long* counter, int64_t* d_results,
                         cudaStream_t st) {
 	DeviceInfo di;
 	fls_status s = device_info(di);
 	if (s != FLS_OK) { return s; }
-	if ((s = cuda_check(cudaMemsetAsync(counter, 0, sizeof(uint32_t), st), "cudaMemsetAsync")) != FLS_OK) { return s; }
+	if ((s = cuda_check(cudaMemsetAsync(counter, 0, sizeof(*counter), st), "cudaMemsetAsync")) != FLS_OK) { return s; }
 	if ((s = cuda_check(cudaMemsetAsync(d_results, 0, sizeof(int64_t) * 2u * b->queries.size(), st), "cudaMemsetAsync")) !=
 	    FLS_OK) {
 		return s;
@@ -300,19 +310,32 @@ fls_status batch_launch(const fls_batch* b, const DevCol* cols, const fls_batch_
 	P.queries    = queries;
 	P.groups     = groups;
 	P.items      = items;
-	P.n_items    = static_cast<uint32_t>(b->items.size());
 	P.counter    = counter;
 	P.results    = reinterpret_cast<long long*>(d_results);
 	P.slot_words = b->slot_words;
 	P.n_slots    = n_slots;
 	P.has_dict   = b->has_dict;
-	// Every SM gets warps: fewer work items than SMs x warps take fewer warps
-	// per CTA, not fewer CTAs (the items are pulled from one counter).
-	const uint64_t n_items = b->items.size();
-	uint64_t       grid64  = std::min<uint64_t>((n_items + warps - 1) / warps, static_cast<uint64_t>(di.sms) * ctas);
+	// Work is handed out in pieces of items, so that a batch of few or short
+	// columns still gives every warp about kPiecesPerWarp of them: an item (64
+	// vectors by default) per warp left 24 columns of 2^14..2^22 values on 3
+	// warps per SM (210 -> 58 us).  Every SM gets warps: fewer pieces
+	// than SMs x warps take fewer warps per CTA, not fewer CTAs.
+	const uint64_t all_warps = static_cast<uint64_t>(di.sms) * ctas * warps;
+	P.piece = static_cast<uint32_t>(std::max<uint64_t>(
+	    1u, std::min<uint64_t>(b->longest, b->vectors / (kPiecesPerWarp * all_warps))));
+	// Every item counts as many pieces as the longest; longer pieces where
+	// that would hand out mostly empty ones.
+	while (P.piece < b->longest && static_cast<uint64_t>((b->longest + P.piece - 1u) / P.piece) * b->items.size() >
+	                                   4u * (b->vectors / P.piece + 1u)) {
+		P.piece = std::min(2u * P.piece, b->longest);
+	}
+	P.pieces_per_item = (b->longest + P.piece - 1u) / P.piece;
+	P.n_pieces        = static_cast<uint64_t>(P.pieces_per_item) * b->items.size();
+	const uint64_t n_work = (b->vectors + P.piece - 1u) / P.piece;
+	uint64_t       grid64 = std::min<uint64_t>((n_work + warps - 1) / warps, static_cast<uint64_t>(di.sms) * ctas);
 	if (grid64 < static_cast<uint64_t>(di.sms)) {
-		grid64 = std::min<uint64_t>(n_items, static_cast<uint64_t>(di.sms));
-		warps  = static_cast<uint32_t>((n_items + grid64 - 1) / grid64);
+		grid64 = std::min<uint64_t>(n_work, static_cast<uint64_t>(di.sms));
+		warps  = static_cast<uint32_t>((n_work + grid64 - 1) / grid64);
 	}
 	const uint32_t grid = static_cast<uint32_t>(grid64);
 	P.warps      = warps;
@@ -370,9 +393,11 @@ fls_status fls_batch_create(const fls_column* cols, uint32_t n_cols, const fls_b
 	}
 	for (uint32_t gi = 0; gi < b->groups.size(); ++gi) {
 		const uint64_t n_vec = (cols[b->groups[gi].col].n_values + 1023u) / 1024u;
+		b->vectors += n_vec;
 		for (uint64_t v = 0; v < n_vec; v += chunk_vectors) {
 			b->items.push_back(make_uint4(gi, static_cast<uint32_t>(v),
 			                              static_cast<uint32_t>(std::min<uint64_t>(n_vec, v + chunk_vectors)), 0u));
+			b->longest = std::max(b->longest, b->items.back().z - b->items.back().y);
 		}
 	}
 	*out = b;
@@ -418,7 +443,7 @@ fls_status fls_batch_run(const fls_batch* b, int64_t* d_results, fls_stream_t st
 	return batch_launch(b, reinterpret_cast<const DevCol*>(w + L.cols),
 	                    reinterpret_cast<const fls_batch_query*>(w + L.queries),
 	                    reinterpret_cast<const BatchGroup*>(w + L.groups), reinterpret_cast<const uint4*>(w + L.items),
-	                    reinterpret_cast<uint32_t*>(w + L.counter), d_results, reinterpret_cast<cudaStream_t>(stream));
+	                    reinterpret_cast<unsigned long long*>(w + L.counter), d_results, reinterpret_cast<cudaStream_t>(stream));
 }
 
 void fls_batch_destroy(fls_batch* b) { delete b; }

@@ -133,3 +133,21 @@ def test_autotuner_join_space(cuda, oracle, tmp_path):
         assert all(np.array_equal(g.cpu().numpy(), want) for g in got)
     finally:
         autotune.reset()
+
+
+@pytest.mark.parametrize("chunk", [1, 3, 64, 1 << 20])
+@pytest.mark.parametrize("lens", [(5,), (1023, 1024, 1025), (64 * 1024, 64 * 1024 + 1, 7), (3_000_001, 2048, 100_000)])
+def test_batch_pieces_of_uneven_items(cuda, chunk, lens):
+    """Items cut into pieces: one vector up to whole columns per item, items of
+    very different length, each run twice."""
+    g = np.random.default_rng(chunk + sum(lens))
+    vals = [g.integers(-500, 1 << 12, n).astype(np.int32) for n in lens]
+    cols = [EncodedColumn.encode(v, i % 2 * 4).to_device() for i, v in enumerate(vals)]  # FOR and DICT
+    qs = [(c, -100 * k, 900 * k, c) for c in range(len(lens)) for k in range(5)]
+    b = Batch(cols, qs, chunk_vectors=chunk)
+    for _ in range(2):
+        got = b.run().cpu().numpy()
+        for i, q in enumerate(qs):
+            assert tuple(got[i]) == _want(vals, q)
+    ops.check_device_error()
+    b.close()
