@@ -4,10 +4,210 @@
 // unpack.cuh:3436), QueryKernel of bitpack_shared_memory.cu:21 /
 // bitpack_register.cu:21 (decode + sum), delta_shared_memory.cu:24 (delta +
 // sum) and delta_global_memory.cu:24 (delta to global memory).
+#include <algorithm>
+
 #include "fls_pipeline.cuh"
 
 namespace fls {
 namespace {
+
+// ------------------------------------------------------- column pipeline
+//
+// One column, vector by vector: warp w of the grid takes vectors w, w + total,
+// ... and keeps a ring of `slots` of them in flight, one bulk copy and one
+// mbarrier each.  Lane l holds the metadata of the warp's l-th next vector
+// (read and checked 32 vectors at a time, the following 32 a window ahead), so
+// a vector costs a few shuffles where a tile of the general pipeline reads,
+// checks and shares its metadata anew (about 200 instructions per tile, of one
+// to three vectors).  50 M values, us before -> after: sum FOR 35 -> 27, DELTA
+// 27 -> 23, RLE 37 -> 33, DICT 62 -> 46; to memory, bound by the writes, RLE 41
+// -> 38, DICT 78 -> 57, FOR and DELTA unchanged at 5.5 TB/s; 4 M values, which
+// now reach every SM, 10.2 -> 8.0 to 8.9.
+struct ColumnCfg {
+	DevCol    col;
+	uint64_t  n_vec, n_values;
+	uint32_t  slots;      // ring depth
+	uint32_t  slot_words; // multiple of 4
+	uint32_t  warps;
+	uint32_t  warp_words; // per-warp region (multiple of 4)
+	uint32_t  dict_off, extra_off, bar_off; // into it
+	uint32_t  has_dict;
+	uint32_t* err;
+};
+
+constexpr uint32_t kMaxSlots = 16; // a window ahead covers any ring
+
+// Metadata of one vector, as a lane holds it.
+struct LaneMeta {
+	uint64_t offset;
+	uint32_t base, packed; // scheme | bw << 8 | aux << 16
+	uint32_t words;        // 0 when nothing is to be copied
+};
+
+// The warp's vectors 32 w .. 32 w + 31: lane l reads and checks the l-th.
+__device__ __forceinline__ LaneMeta load_window(const ColumnCfg& cfg, uint64_t first, uint64_t total, uint64_t w,
+                                                uint32_t lane) {
+	LaneMeta       m {0, 0, kBadScheme, 0};
+	const uint64_t v = first + (32u * w + lane) * total;
+	if (v < cfg.n_vec) {
+		VecInfo vi {};
+		bool    ok = dev::vec_info(cfg.col, v, dev::load_meta(cfg.col, v), vi);
+		// RLE / DICT vectors need the dictionary scratch
+		ok = ok && (cfg.has_dict || (vi.scheme != FLS_SCHEME_RLE && vi.scheme != FLS_SCHEME_DICT));
+		if (ok) {
+			m = LaneMeta {vi.offset, static_cast<uint32_t>(vi.base), vi.scheme | (vi.bw << 8) | (vi.aux << 16), vi.words};
+		} else {
+			raise_err(cfg.err, kErrBadMeta);
+		}
+	}
+	return m;
+}
+
+// Copies the vector held by lane `src` into a slot.  Words is a multiple of 4
+// and the offset too (checked), so the copy's ends are 16-byte aligned.
+__device__ __forceinline__ void issue_vector(const ColumnCfg& cfg, uint32_t* slot, uint64_t* bar, const LaneMeta& m,
+                                             uint32_t src, uint32_t lane, uint64_t pol) {
+	if (lane == src) {
+		dev::mbar_arrive_expect_tx(bar, 4u * m.words);
+		if (m.words) { dev::bulk_g2s(slot, cfg.col.data + m.offset, 4u * m.words, bar, pol); }
+	}
+}
+
+// The operator's view of a staged vector.
+struct ColumnVec {
+	VecInfo         vi;
+	const uint32_t* s;
+	uint32_t*       dict;
+	uint32_t*       extra;
+	uint64_t        v;
+	__device__ uint32_t rows(const ColumnCfg& cfg, uint32_t lane) const {
+		const uint64_t start = v * 1024u;
+		if (start + 1024u <= cfg.n_values) { return 0xffffffffu; }
+		return dev::tail_rows(cfg.col.layout, lane, static_cast<uint32_t>(cfg.n_values - start));
+	}
+};
+
+template <class Op>
+__global__ void __launch_bounds__(Op::kWarps * 32, 1)
+    column_kernel(const __grid_constant__ ColumnCfg cfg, const __grid_constant__ Op op) {
+	extern __shared__ __align__(128) uint32_t smem[];
+	const uint32_t     lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	uint32_t*          base = smem + warp * cfg.warp_words;
+	uint64_t*          bars = reinterpret_cast<uint64_t*>(base + cfg.bar_off);
+	typename Op::State state {};
+	const uint64_t     total = static_cast<uint64_t>(gridDim.x) * cfg.warps;
+	const uint64_t     first = static_cast<uint64_t>(blockIdx.x) * cfg.warps + warp;
+	const uint64_t     n     = first < cfg.n_vec ? (cfg.n_vec - first + total - 1u) / total : 0u;
+	LaneMeta           now = load_window(cfg, first, total, 0, lane), next = load_window(cfg, first, total, 1, lane);
+	if (lane < cfg.slots) { dev::mbar_init(bars + lane, 1); }
+	dev::fence_mbar_init();
+	__syncwarp();
+	const uint64_t pol = dev::l2_evict_first_policy();
+	for (uint32_t q = 0; q < cfg.slots && q < n; ++q) {
+		issue_vector(cfg, base + q * cfg.slot_words, bars + q, now, q, lane, pol);
+	}
+	uint32_t slot = 0, phase = 0;
+	for (uint64_t q = 0; q < n; ++q) {
+		const uint32_t j = static_cast<uint32_t>(q) & 31u;
+		if (j == 0 && q != 0) {
+			now  = next;
+			next = load_window(cfg, first, total, (q >> 5) + 1u, lane);
+		}
+		if (!dev::mbar_wait_bounded(bars + slot, phase, kWaitPolls)) {
+			raise_err(cfg.err, kErrTimeout);
+			// Give the copies still in flight a bounded chance to land before exit.
+			for (uint32_t s = 0; s < cfg.slots; ++s) {
+				dev::mbar_wait_bounded(bars + s, phase, 1u << 10);
+				dev::mbar_wait_bounded(bars + s, phase ^ 1u, 1u << 10);
+			}
+			return;
+		}
+		const uint32_t packed = __shfl_sync(0xffffffffu, now.packed, j);
+		ColumnVec      cv;
+		cv.vi.base   = static_cast<int32_t>(__shfl_sync(0xffffffffu, now.base, j));
+		cv.vi.scheme = packed & 0xffu;
+		cv.vi.bw     = (packed >> 8) & 0xffu;
+		cv.vi.aux    = packed >> 16;
+		cv.s         = base + slot * cfg.slot_words;
+		cv.dict      = base + cfg.dict_off;
+		cv.extra     = base + cfg.extra_off;
+		cv.v         = first + q * total;
+		if (cv.vi.scheme != kBadScheme) { op.process(state, cv, lane, cfg); }
+		__syncwarp();
+		if (q + cfg.slots < n) {
+			dev::fence_proxy_async_smem();
+			const uint32_t ahead = j + cfg.slots; // below 64
+			issue_vector(cfg, base + slot * cfg.slot_words, bars + slot, ahead < 32u ? now : next, ahead & 31u, lane, pol);
+		}
+		if (++slot == cfg.slots) {
+			slot = 0;
+			phase ^= 1u;
+		}
+	}
+	op.finish(state, lane, cfg);
+}
+
+// Lays out and launches: as many warps as the operator takes and shared
+// memory holds at two slots or more, then slots up to the launch
+// configuration's bytes in flight per warp (stages x tile bytes), or a third
+// of them where every vector is also written out: past that the reads in
+// flight only disturb the writes (50 M values to memory, FOR of mixed widths:
+// 49.7 us at 4 KB a warp, 52.3 at 12 KB; DELTA 45.0 and 46.5).  A column of
+// fewer vectors than warps spreads over the SMs.
+template <class Op>
+fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_words, cudaStream_t stream) {
+	ColumnCfg  cfg {};
+	DeviceInfo di;
+	fls_status s = device_info(di);
+	if (s != FLS_OK) { return s; }
+	if ((s = make_devcol(col, cfg.col)) != FLS_OK) { return s; }
+	uint32_t warps = 0, stages = 0, ctas = 0, tile_bytes = 0;
+	fls_get_launch_config(&warps, &stages, &ctas, &tile_bytes);
+	warps        = std::min(warps, Op::kWarps);
+	cfg.has_dict = col.meta && (col.scheme_mask & ((1u << FLS_SCHEME_RLE) | (1u << FLS_SCHEME_DICT))) ? 1u : 0u;
+	cfg.n_values = col.n_values;
+	cfg.n_vec    = (col.n_values + 1023u) / 1024u;
+	const auto round4 = [](uint32_t w) { return (w + 3u) & ~3u; };
+	cfg.slot_words    = round4(cfg.col.slot_words);
+	const uint32_t flight = stages * tile_bytes / Op::kFlightShare;
+	const uint32_t want   = std::max<uint32_t>(1u, flight / std::max<uint32_t>(4u * cfg.slot_words, 256u));
+	const uint32_t fixed = kSlotSlackWords + (cfg.has_dict ? kDictWords : 0u) + round4(extra_words) + 2u * kMaxSlots;
+	const uint32_t avail = static_cast<uint32_t>(di.max_smem) / 4u;
+	const auto     fits  = [&](uint32_t w, uint32_t slots) { return w * (slots * cfg.slot_words + fixed) <= avail; };
+	while (warps > 1 && !fits(warps, 2)) { --warps; }
+	if (!fits(warps, 1)) { return set_error(FLS_ERR_CAPACITY, "vectors too large for shared-memory staging"); }
+	cfg.slots = std::min<uint32_t>(std::max<uint32_t>(want, 2u), kMaxSlots);
+	while (cfg.slots > 1 && !fits(warps, cfg.slots)) { --cfg.slots; }
+	uint64_t grid = std::min<uint64_t>((cfg.n_vec + warps - 1u) / warps, static_cast<uint64_t>(di.sms) * ctas);
+	if (grid < static_cast<uint64_t>(di.sms)) {
+		grid  = std::min<uint64_t>(cfg.n_vec, static_cast<uint64_t>(di.sms));
+		warps = static_cast<uint32_t>((cfg.n_vec + grid - 1u) / grid);
+	}
+	cfg.warps      = warps;
+	cfg.dict_off   = cfg.slots * cfg.slot_words + kSlotSlackWords;
+	cfg.extra_off  = cfg.dict_off + (cfg.has_dict ? kDictWords : 0u);
+	cfg.bar_off    = cfg.extra_off + round4(extra_words);
+	cfg.warp_words = cfg.bar_off + 2u * kMaxSlots;
+	cfg.err        = device_error_word(stream);
+	{
+		static std::mutex mu;
+		static uint64_t   configured = 0; // bit d: device d's shared-memory attribute raised
+		int               dev        = 0;
+		cudaGetDevice(&dev);
+		std::lock_guard<std::mutex> lk(mu);
+		if (dev >= 64 || !(configured & (1ull << dev))) {
+			s = cuda_check(cudaFuncSetAttribute(column_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem),
+			               "cudaFuncSetAttribute");
+			if (s != FLS_OK) { return s; }
+			if (dev < 64) { configured |= 1ull << dev; }
+		}
+	}
+	column_kernel<Op><<<static_cast<uint32_t>(grid), 32u * warps, 4ull * cfg.warp_words * warps, stream>>>(cfg, op);
+	count_launch();
+	return cuda_check(cudaGetLastError(), "column_kernel launch");
+}
+
+// -------------------------------------------------------------- operators
 
 struct NoState {};
 
@@ -16,19 +216,16 @@ struct NoState {};
 // padded shared-memory tile (33 words per chunk, conflict-free) into original
 // order.
 struct DecodeOp {
+	static constexpr uint32_t kWarps = 16, kFlightShare = 3;
 	using State = NoState;
 	uint32_t* out;
 	uint32_t  original;
-	__device__ void cta_setup(State&, uint32_t*, const StageCfg&) const {}
-	__device__ void process(State&, uint64_t v, const WarpStage& ws, uint32_t st, uint32_t i, uint32_t lane,
-	                        const StageCfg&) const {
-		const StagedVec sv = staged(ws, st, i, 0);
-		if (sv.bad()) { return; }
+	__device__ void process(State&, const ColumnVec& cv, uint32_t lane, const ColumnCfg&) const {
 		uint32_t vals[32];
-		dev::decode_vals(sv.s, sv.vi, ws.dict(), lane, vals);
-		uint32_t* dst = out + v * 1024u;
+		dev::decode_vals(cv.s, cv.vi, cv.dict, lane, vals);
+		uint32_t* dst = out + cv.v * 1024u;
+		uint32_t* tb  = cv.extra;
 		if (original) {
-			uint32_t*      tb = ws.extra();
 			const uint32_t cb = 33u * dev::chunk_of_lane(lane);
 #pragma unroll
 			for (uint32_t r = 0; r < 32; ++r) { tb[cb + dev::step_of_row(r)] = vals[r]; }
@@ -41,7 +238,7 @@ struct DecodeOp {
 			for (uint32_t r = 0; r < 32; ++r) { dev::st_stream(dst + 32u * r + lane, vals[r]); }
 		}
 	}
-	__device__ void finish(State&, uint32_t, const StageCfg&) const {}
+	__device__ void finish(State&, uint32_t, const ColumnCfg&) const {}
 };
 
 struct AccState {
@@ -51,17 +248,14 @@ struct AccState {
 // Decode fused with a uint64 sum; four independent partial sums per lane, one
 // atomic per warp at the end.
 struct DecodeSumOp {
+	static constexpr uint32_t kWarps = 16, kFlightShare = 1;
 	using State = AccState;
 	unsigned long long* sum;
-	__device__ void cta_setup(State&, uint32_t*, const StageCfg&) const {}
-	__device__ void process(State& S, uint64_t v, const WarpStage& ws, uint32_t st, uint32_t i, uint32_t lane,
-	                        const StageCfg& cfg) const {
-		const StagedVec sv = staged(ws, st, i, 0);
-		if (sv.bad()) { return; }
+	__device__ void process(State& S, const ColumnVec& cv, uint32_t lane, const ColumnCfg& cfg) const {
 		uint32_t vals[32];
 		// Values are summed as uint32 (base added per value: it may wrap).
-		dev::decode_vals(sv.s, sv.vi, ws.dict(), lane, vals);
-		const uint32_t     m = valid_rows(cfg, v, lane);
+		dev::decode_vals(cv.s, cv.vi, cv.dict, lane, vals);
+		const uint32_t     m = cv.rows(cfg, lane);
 		unsigned long long p[4] = {0, 0, 0, 0};
 		if (m == 0xffffffffu) { // every vector but the column's last
 #pragma unroll
@@ -72,7 +266,7 @@ struct DecodeSumOp {
 		}
 		S.acc += (p[0] + p[1]) + (p[2] + p[3]);
 	}
-	__device__ void finish(State& S, uint32_t lane, const StageCfg&) const {
+	__device__ void finish(State& S, uint32_t lane, const ColumnCfg&) const {
 		const unsigned long long s = warp_sum_u64(S.acc);
 		if (lane == 0 && s) { atomicAdd(sum, s); }
 	}
@@ -202,47 +396,13 @@ __device__ __forceinline__ unsigned long long dict_lane_sum(const uint32_t* __re
 	return Small ? static_cast<unsigned long long>(s32) : s64;
 }
 
-// Sequentially FOR-packed dictionary of n entries at bit width BW into dst
-// (base added), lanes striding over the entries.
-template <int BW>
-__device__ __forceinline__ void unpack_dict_bw(const uint32_t* __restrict__ src, uint32_t n, int32_t base,
-                                               uint32_t* __restrict__ dst, uint32_t lane) {
-	const uint32_t b = static_cast<uint32_t>(base);
-	for (uint32_t k = lane; k < n; k += 32) {
-		uint32_t v = 0;
-		if constexpr (BW == 32) {
-			v = src[k];
-		} else if constexpr (BW > 0) {
-			const uint32_t bit = k * BW, w = bit >> 5, sh = bit & 31u;
-			const uint32_t hi  = (sh + BW > 32u) ? src[w + 1] : 0u; // never past the dictionary
-			v                  = __funnelshift_r(src[w], hi, sh) & ((1u << BW) - 1u);
-		}
-		dst[k] = v + b;
-	}
-	__syncwarp();
-}
-
-__device__ __forceinline__ void unpack_dict_any(const uint32_t* __restrict__ src, uint32_t n, uint32_t bw,
-                                                int32_t base, uint32_t* __restrict__ dst, uint32_t lane) {
-	switch (bw) {
-#define FLS_DICT_UNPACK(B)                                                                                             \
-	case B: unpack_dict_bw<B>(src, n, base, dst, lane); break;
-		FLS_BW_CASES_0_32(FLS_DICT_UNPACK)
-#undef FLS_DICT_UNPACK
-	default: break;
-	}
-}
-
 template <uint32_t SCHEME>
 struct SchemeSumOp {
+	static constexpr uint32_t kWarps = 16, kFlightShare = 1;
 	using State = AccState;
 	unsigned long long* sum;
-	__device__ void cta_setup(State&, uint32_t*, const StageCfg&) const {}
-	__device__ void process(State& S, uint64_t v, const WarpStage& ws, uint32_t st, uint32_t i, uint32_t lane,
-	                        const StageCfg& cfg) const {
-		const StagedVec sv = staged(ws, st, i, 0);
-		if (sv.bad()) { return; }
-		const uint32_t rows = valid_rows(cfg, v, lane);
+	__device__ void process(State& S, const ColumnVec& sv, uint32_t lane, const ColumnCfg& cfg) const {
+		const uint32_t rows = sv.rows(cfg, lane);
 		if (sv.vi.scheme != SCHEME) { // the host saw one scheme; any other vector is flagged, not read
 			if (lane == 0) { raise_err(cfg.err, kErrBadMeta); }
 			return;
@@ -256,8 +416,8 @@ struct SchemeSumOp {
 			default: break;
 			}
 		} else if constexpr (SCHEME == FLS_SCHEME_RLE) {
-			uint32_t* dict = ws.dict();
-			unpack_dict_any(sv.s + 48, sv.vi.aux, sv.vi.bw, sv.vi.base, dict, lane);
+			uint32_t* dict = sv.dict;
+			dev::unpack_dict(sv.s + 48, sv.vi.aux, sv.vi.bw, sv.vi.base, dict, lane);
 			if (__all_sync(0xffffffffu, rows == 0xffffffffu)) {
 				S.acc += small_values(sv.vi) ? rle_lane_sum<true, true>(sv.s, dict, lane, rows)
 				                             : rle_lane_sum<false, true>(sv.s, dict, lane, rows);
@@ -267,9 +427,9 @@ struct SchemeSumOp {
 			}
 			__syncwarp();
 		} else {
-			uint32_t*      dict = ws.dict();
+			uint32_t*      dict = sv.dict;
 			const uint32_t cbw  = dev::bits_of(sv.vi.aux - 1u);
-			unpack_dict_any(sv.s + 32u * cbw, sv.vi.aux, sv.vi.bw, sv.vi.base, dict, lane);
+			dev::unpack_dict(sv.s + 32u * cbw, sv.vi.aux, sv.vi.bw, sv.vi.base, dict, lane);
 			const bool small = small_values(sv.vi);
 			if (!__all_sync(0xffffffffu, rows == 0xffffffffu)) {
 				S.acc += dict_lane_sum_rows(sv.s, dict, lane, cbw, rows);
@@ -285,7 +445,7 @@ struct SchemeSumOp {
 			__syncwarp();
 		}
 	}
-	__device__ void finish(State& S, uint32_t lane, const StageCfg&) const {
+	__device__ void finish(State& S, uint32_t lane, const ColumnCfg&) const {
 		const unsigned long long s = warp_sum_u64(S.acc);
 		if (lane == 0 && s) { atomicAdd(sum, s); }
 	}
@@ -312,50 +472,39 @@ extern "C" {
 fls_status fls_decode_u32(const fls_column* col, uint32_t* d_out, uint32_t order, fls_stream_t stream) {
 	if (!col || !d_out) { return set_error(FLS_ERR_INVALID_ARG, "fls_decode_u32: null pointer"); }
 	if (order > FLS_ORDER_ORIGINAL) { return set_error(FLS_ERR_INVALID_ARG, "fls_decode_u32: bad order"); }
-	StageCfg   cfg;
-	uint32_t   grid, threads;
-	size_t     smem;
-	const bool orig = order == FLS_ORDER_ORIGINAL && col->layout == FLS_LAYOUT_TRANSPOSED;
-	fls_status s    = plan_stages(col, 1, orig ? kTBufWords : 0u, 0u, cfg, grid, threads, smem);
-	if (s != FLS_OK) { return s; }
-	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+	const bool   orig = order == FLS_ORDER_ORIGINAL && col->layout == FLS_LAYOUT_TRANSPOSED;
+	cudaStream_t st   = reinterpret_cast<cudaStream_t>(stream);
 	if (tuning_jit() && !orig) {
-		bool used = false;
-		s         = jit_decode(col, 1, d_out, nullptr, st, used);
+		bool       used = false;
+		fls_status s    = jit_decode(col, 1, d_out, nullptr, st, used);
 		if (s != FLS_OK || used) { return s; }
 	}
 	DecodeOp op {};
 	op.out      = d_out;
 	op.original = orig ? 1u : 0u;
-	return launch_staged(cfg, op, grid, threads, smem, st);
+	return launch_column(*col, op, orig ? kTBufWords : 0u, st);
 }
 
 fls_status fls_decode_sum_u32(const fls_column* col, uint64_t* d_sum, fls_stream_t stream) {
 	if (!col || !d_sum) { return set_error(FLS_ERR_INVALID_ARG, "fls_decode_sum_u32: null pointer"); }
-	StageCfg   cfg;
-	uint32_t   grid, threads;
-	size_t     smem;
-	fls_status s = plan_stages(col, 1, 0u, 0u, cfg, grid, threads, smem);
+	DevCol     checked;
+	fls_status s = make_devcol(*col, checked);
 	if (s != FLS_OK) { return s; }
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 	if ((s = cuda_check(cudaMemsetAsync(d_sum, 0, sizeof(uint64_t), st), "cudaMemsetAsync")) != FLS_OK) { return s; }
+	auto* sum = reinterpret_cast<unsigned long long*>(d_sum);
 	if (tuning_jit()) {
 		bool used = false;
 		s         = jit_decode(col, 0, nullptr, d_sum, st, used);
 		if (s != FLS_OK || used) { return s; }
-	}
-	if (tuning_jit()) {
-		auto* sum = reinterpret_cast<unsigned long long*>(d_sum);
 		switch (single_scheme(*col)) {
-		case FLS_SCHEME_DELTA: return launch_staged(cfg, SchemeSumOp<FLS_SCHEME_DELTA> {sum}, grid, threads, smem, st);
-		case FLS_SCHEME_RLE: return launch_staged(cfg, SchemeSumOp<FLS_SCHEME_RLE> {sum}, grid, threads, smem, st);
-		case FLS_SCHEME_DICT: return launch_staged(cfg, SchemeSumOp<FLS_SCHEME_DICT> {sum}, grid, threads, smem, st);
+		case FLS_SCHEME_DELTA: return launch_column(*col, SchemeSumOp<FLS_SCHEME_DELTA> {sum}, 0u, st);
+		case FLS_SCHEME_RLE: return launch_column(*col, SchemeSumOp<FLS_SCHEME_RLE> {sum}, 0u, st);
+		case FLS_SCHEME_DICT: return launch_column(*col, SchemeSumOp<FLS_SCHEME_DICT> {sum}, 0u, st);
 		default: break;
 		}
 	}
-	DecodeSumOp op {};
-	op.sum = reinterpret_cast<unsigned long long*>(d_sum);
-	return launch_staged(cfg, op, grid, threads, smem, st);
+	return launch_column(*col, DecodeSumOp {sum}, 0u, st);
 }
 
 } // extern "C"

@@ -181,3 +181,29 @@ def test_argument_validation(cuda):
     d.desc.bw = 31  # larger than the data buffer allows
     with pytest.raises(FlsError):
         ops.query_aggregate(d)
+
+
+@pytest.mark.parametrize("n_vec", [1, 147, 149, 148 * 32 - 1, 148 * 33 + 1, 148 * 64 + 3])
+@pytest.mark.parametrize("scheme", [0, 1, 2, 4])
+def test_column_windows_and_rings(cuda, n_vec, scheme):
+    """One warp per SM (148): its metadata windows (32 vectors) and rings begin,
+    wrap and end at every count around them; a column of one scheme and one
+    with another scheme in between, summed and decoded in both orders."""
+    import torch
+    from fastlanesgpu_b200.column import encode_column_gpu
+    n = n_vec * 1024 - 5
+    v = torch.from_numpy(datagen.geometric_runs(n, mean_run=8.0, value_bits=12, seed=n_vec)).cuda()
+    if scheme == 1:
+        v = torch.cumsum(v, 0).to(torch.int32)
+    mixed = torch.full((n_vec,), scheme, dtype=torch.uint8, device="cuda")
+    mixed[::3] = (scheme + 1) % 3
+    ops.set_launch_config(1, 2, 1, 2048)
+    try:
+        for col in (encode_column_gpu(v, scheme), encode_column_gpu(v, mixed)):
+            assert torch.equal(ops.unpack_global(col, ORDER_ORIGINAL)[:n], v)
+            stored = ops.unpack_global(col, ORDER_STORED)
+            assert int(ops.query_aggregate(col).cpu()[0]) == int((v.long() & 0xFFFFFFFF).sum())
+            assert int((stored.long() & 0xFFFFFFFF).sum()) == int((v.long() & 0xFFFFFFFF).sum()) + 5 * (int(v[-1]) & 0xFFFFFFFF)
+        ops.check_device_error()
+    finally:
+        ops.set_launch_config()
