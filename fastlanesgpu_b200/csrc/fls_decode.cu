@@ -487,8 +487,10 @@ fls_status fls_decode_u32(const fls_column* col, uint32_t* d_out, uint32_t order
 
 fls_status fls_decode_sum_u32(const fls_column* col, uint64_t* d_sum, fls_stream_t stream) {
 	if (!col || !d_sum) { return set_error(FLS_ERR_INVALID_ARG, "fls_decode_sum_u32: null pointer"); }
+	DeviceInfo di;
 	DevCol     checked;
-	fls_status s = make_devcol(*col, checked);
+	fls_status s = device_info(di);
+	if (s == FLS_OK) { s = make_devcol(*col, checked); }
 	if (s != FLS_OK) { return s; }
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 	if ((s = cuda_check(cudaMemsetAsync(d_sum, 0, sizeof(uint64_t), st), "cudaMemsetAsync")) != FLS_OK) { return s; }
