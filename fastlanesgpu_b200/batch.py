@@ -5,13 +5,8 @@ from __future__ import annotations
 
 import ctypes
 
-from ._lib import BatchQuery, check, lib
+from ._lib import BatchQuery, check, lib, stream_handle as _stream
 from .column import columns_array
-
-
-def _stream():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
 
 
 class Batch:

@@ -241,7 +241,7 @@ def encode_column_gpu(values, schemes=0, layout: int = LAYOUT_TRANSPOSED, round4
     bound = int(lib().fls_encode_bound_words(n))
     out = torch.empty(bound + 4, dtype=torch.int32, device=dev)
     meta = torch.empty(nv * 4, dtype=torch.int32, device=dev)
-    info = torch.zeros(3, dtype=torch.int64, device=dev)
+    info = torch.empty(3, dtype=torch.int64, device=dev)  # the call sets all three words
     ws_bytes = int(lib().fls_encode_gpu_workspace_bytes(n))
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     per_vec = not isinstance(schemes, (int, np.integer))
@@ -250,8 +250,8 @@ def encode_column_gpu(values, schemes=0, layout: int = LAYOUT_TRANSPOSED, round4
     check(lib().fls_encode_column_gpu(values.data_ptr(), n, schemes.data_ptr() if per_vec else None,
                                       0 if per_vec else int(schemes), layout, int(round4), out.data_ptr(), bound + 4,
                                       meta.data_ptr(), info.data_ptr(), ws.data_ptr(), ws_bytes,
-                                      torch.cuda.current_stream().cuda_stream), "fls_encode_column_gpu")
-    total, mx, mask = (int(x) for x in info.cpu())
+                                      _lib.stream_handle()), "fls_encode_column_gpu")
+    total, mx, mask = info.tolist()
     if compact:
         out = out[:max(total, 4)].clone()
     return DeviceEncodedColumn(out, meta, n, layout, total, mx, mask)
@@ -264,11 +264,25 @@ class PendingEncode:
     be encoded back to back with no host round trip in between."""
 
     def __init__(self, out, meta, info, schemes, n, layout, compact):
+        import torch
         self.out, self.meta, self.info, self.schemes = out, meta, info, schemes
         self.n, self.layout, self.compact = n, layout, compact
+        # The info words start on their way to the host right behind the
+        # encode, so finish() waits for this encode only and not for the ones
+        # enqueued after it.  (Not while capturing: finish() then reads them.)
+        self._host = self._done = None
+        if not torch.cuda.is_current_stream_capturing():
+            self._host = torch.empty(4, dtype=torch.int64, pin_memory=True)
+            self._host.copy_(info, non_blocking=True)
+            self._done = torch.cuda.Event()
+            self._done.record()
 
     def finish(self):
-        total, mx, mask, n_fb = (int(x) for x in self.info.cpu())
+        if self._done is not None:
+            self._done.synchronize()
+            total, mx, mask, n_fb = self._host.tolist()
+        else:
+            total, mx, mask, n_fb = self.info.tolist()
         out = self.out[:max(total, 4)].clone() if self.compact else self.out
         return DeviceEncodedColumn(out, self.meta, self.n, self.layout, total, mx, mask), self.schemes, n_fb
 
@@ -294,7 +308,7 @@ def encode_column_learned_gpu(values, params, threshold: float = 0.9, kappa: flo
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
     check(lib().fls_encode_learned_gpu(values.data_ptr(), n, params.data_ptr(), threshold, kappa, layout,
                                        out.data_ptr(), bound + 4, meta.data_ptr(), info.data_ptr(), schemes.data_ptr(),
-                                       ws.data_ptr(), ws_bytes, torch.cuda.current_stream().cuda_stream),
+                                       ws.data_ptr(), ws_bytes, _lib.stream_handle()),
           "fls_encode_learned_gpu")
     pending = PendingEncode(out, meta, info, schemes, n, layout, compact)
     return pending if defer else pending.finish()

@@ -794,6 +794,20 @@ fls_status fls_pht_build_ranges(const int32_t* d_filter, int32_t lo0, int32_t hi
 	return cuda_check(cudaGetLastError(), "pht_build_kernel launch");
 }
 
+fls_status fls_pht_build_zeroed(const int32_t* d_filter, int32_t lo0, int32_t hi0, int32_t lo1, int32_t hi1,
+                                const int32_t* d_keys, const int32_t* d_vals, uint64_t n, int32_t* d_ht,
+                                int32_t ht_len, int32_t keys_min, fls_stream_t stream) {
+	if (!d_keys || !d_ht || ht_len <= 0) { return set_error(FLS_ERR_INVALID_ARG, "fls_pht_build: bad arguments"); }
+	DeviceInfo di;
+	fls_status s = device_info(di);
+	if (s != FLS_OK) { return s; }
+	const size_t slots = static_cast<size_t>(ht_len) * (d_vals ? 2u : 1u);
+	s = cuda_check(cudaMemsetAsync(d_ht, 0, sizeof(int32_t) * slots, reinterpret_cast<cudaStream_t>(stream)),
+	               "cudaMemsetAsync");
+	if (s != FLS_OK) { return s; }
+	return fls_pht_build_ranges(d_filter, lo0, hi0, lo1, hi1, d_keys, d_vals, n, d_ht, ht_len, keys_min, stream);
+}
+
 uint64_t fls_join_workspace_bytes(const fls_join_groupby_desc* desc) {
 	return check_groupby_desc(desc) == FLS_OK ? jit_probe_workspace_bytes(desc) : 0u;
 }

@@ -24,13 +24,8 @@ import ctypes
 import numpy as np
 
 from ._lib import (MAX_FILTERS, MAX_GROUP_KEYS, MAX_PROBES, ORDER_STORED, Column, FilterAggDesc, JitStats, JoinAggDesc,
-                   JoinGroupbyDesc, check, lib)
+                   JoinGroupbyDesc, check, lib, stream_handle as _stream)
 from .column import DeviceColumn, columns_array
-
-
-def _stream():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _p(a: np.ndarray) -> int:
@@ -189,17 +184,17 @@ def build_pht(keys, ht_len: int, vals=None, filt=None, filter_eq: int = 1, keys_
     import torch
     size = ht_len if vals is None else 2 * ht_len
     if out is None:
-        out = torch.zeros(size, dtype=torch.int32, device=keys.device)
-    else:
-        out.zero_()
+        out = torch.empty(size, dtype=torch.int32, device=keys.device)
+    elif out.numel() != size or out.dtype != torch.int32 or not out.is_contiguous():
+        out.zero_()  # the library zeroes the ht_len slots of a table that is just as large
     if ranges is None:
         ranges = [(filter_eq, filter_eq)]
     if not 1 <= len(ranges) <= 2:
         raise ValueError("one or two filter ranges")
     (lo0, hi0), (lo1, hi1) = ranges[0], ranges[1] if len(ranges) == 2 else (1, 0)
-    check(lib().fls_pht_build_ranges(0 if filt is None else filt.data_ptr(), lo0, hi0, lo1, hi1, keys.data_ptr(),
+    check(lib().fls_pht_build_zeroed(0 if filt is None else filt.data_ptr(), lo0, hi0, lo1, hi1, keys.data_ptr(),
                                      0 if vals is None else vals.data_ptr(), keys.numel(), out.data_ptr(), ht_len,
-                                     keys_min, _stream()), "fls_pht_build_ranges")
+                                     keys_min, _stream()), "fls_pht_build_zeroed")
     return out
 
 

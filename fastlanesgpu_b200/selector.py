@@ -17,7 +17,7 @@ import time
 import numpy as np
 
 from . import datagen
-from ._lib import MLP_IN, MLP_N_PARAMS, check, lib
+from ._lib import MLP_IN, MLP_N_PARAMS, check, lib, stream_handle as _stream
 from .ops import encode_exhaustive
 
 N_SCHEMES = 5
@@ -36,11 +36,6 @@ def decode_aware_labels(sizes: np.ndarray, kappa: float = 0.0) -> np.ndarray:
     cost[sizes == 0xFFFFFFFF] = np.inf
     order = np.argsort(DECODE_COST, kind="stable")  # cheapest decode first wins ties
     return order[np.argmin(cost[:, order], axis=1)].astype(np.uint8)
-
-
-def _stream():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
 
 
 def gpu_features(values_dev) -> "torch.Tensor":

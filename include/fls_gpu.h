@@ -323,6 +323,11 @@ fls_status fls_pht_build(const int32_t* d_filter, int32_t filter_eq, const int32
 fls_status fls_pht_build_ranges(const int32_t* d_filter, int32_t lo0, int32_t hi0, int32_t lo1, int32_t hi1,
                                 const int32_t* d_keys, const int32_t* d_vals, uint64_t n, int32_t* d_ht,
                                 int32_t ht_len, int32_t keys_min, fls_stream_t stream);
+/* fls_pht_build_ranges into a table that need not be zeroed: the call zeroes
+ * its slots first, in stream order. */
+fls_status fls_pht_build_zeroed(const int32_t* d_filter, int32_t lo0, int32_t hi0, int32_t lo1, int32_t hi1,
+                                const int32_t* d_keys, const int32_t* d_vals, uint64_t n, int32_t* d_ht,
+                                int32_t ht_len, int32_t keys_min, fls_stream_t stream);
 
 typedef struct fls_probe {
 	uint32_t       col;      /* probed foreign-key column                        */
