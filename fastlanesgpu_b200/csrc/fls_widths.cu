@@ -10,7 +10,7 @@
 // each 128-byte row, which holds 32/T consecutive lanes, and extracts row r
 // of all of them at once (SIMD within a register: every lane of a word has
 // the same bit offset r*bw, so one shift and a per-lane mask serve all; the
-// base is added lane-wise without carries between lanes).  64-bit lanes: a
+// base is added lane-wise without carries between lanes), at constant widths.  64-bit lanes: a
 // half-warp per vector, one lane per thread.  Both read and write 128-byte
 // rows per instruction.
 #include <cuda_runtime.h>
@@ -41,34 +41,64 @@ __device__ __forceinline__ uint32_t lane_sum(uint32_t x) {
 	}
 }
 
-// One vector of 8/16-bit lanes: row r of the 32/B lanes of thread word t.
-// OUT / SUM: write the values / add them to part; TAIL: the column's last,
-// partial vector (rem values).  NOWRAP (sum only, whole vectors): the host
-// proved base + 2^bw - 1 < 2^B, so no value wraps and the packed fields are
-// summed in 2B-bit halves with the base added once per thread (32 values).
-// Branch-free per row, so the loads of all rows can issue before the first
-// is used.
-template <int B, bool OUT, bool SUM, bool TAIL, bool NOWRAP = false>
-__device__ __forceinline__ void narrow_vector(const uint32_t* __restrict src, uint32_t* __restrict dst, uint32_t bw,
-                                              uint32_t vm, uint32_t base_rep, uint32_t t, uint64_t rem,
-                                              uint32_t& part) {
+// The block's sum into the result with one atomic: one per warp, 18,944 on one
+// address, took 5 of the 17 us of 90 M 8-bit values at width 3.
+__device__ __forceinline__ void add_block_sum(unsigned long long acc, unsigned long long* sum) {
+	__shared__ unsigned long long part[8];
+	const uint32_t lane = threadIdx.x & 31u;
+	acc                 = warp_sum_u64(acc);
+	if (lane == 0) { part[threadIdx.x >> 5] = acc; }
+	__syncthreads();
+	if (threadIdx.x < 32u) {
+		acc = warp_sum_u64(lane < 8u ? part[lane] : 0ull);
+		if (lane == 0 && acc) { atomicAdd(sum, acc); }
+	}
+}
+
+// One vector of 8/16-bit lanes at width BW: rows of the 32/B lanes of thread
+// word t.  OUT / SUM: write the values / add them to part; TAIL: the column's
+// last, partial vector (rem values).  NOWRAP: the host proved base + 2^bw - 1 <
+// 2^B, so no value wraps: a packed add gives the values, and whole vectors sum
+// their fields packed (while 2^B holds a thread's rows of them) or in 2B-bit
+// halves, with the base added once per thread (32 values).
+//
+// With the width a constant every shift and mask is one too and a thread
+// reads its BW words once: about 6 instructions per row, 37 with the width at
+// run time (two clamped reads per row among them).  90 M values, us before ->
+// after: to memory 8-bit at width 3 33 -> 23, 16-bit at width 5 59 -> 41 and 13
+// 66 -> 54 (write bound); sums 8-bit at width 3 35 -> 16, 16-bit at width 5 61
+// -> 20 and 13 63 -> 30.
+template <int B, int BW, bool OUT, bool SUM, bool TAIL, bool NOWRAP>
+__device__ __forceinline__ void narrow_vector(const uint32_t* __restrict src, uint32_t* __restrict dst,
+                                              uint32_t base_rep, uint32_t t, uint64_t rem, uint32_t& part) {
 	using N              = Narrow<B>;
 	constexpr uint32_t L = 32u / B;   // lanes per thread word
 	constexpr uint32_t S = 1024u / B; // lanes per vector
-	const uint32_t     last = bw ? bw - 1u : 0u;
-	static_assert(!NOWRAP || (SUM && !OUT && !TAIL), "NOWRAP sums whole vectors only");
-	uint32_t           ev = 0, od = 0; // NOWRAP: even and odd lanes' fields, 2B-bit sums
+	constexpr uint32_t V = (1u << BW) - 1u;
+	constexpr bool     kFields = SUM && !TAIL && NOWRAP;         // fields are summed, not values
+	constexpr bool     kPacked = BW + (B == 8 ? 3 : 4) <= B;     // B rows of them fit a lane
+	uint32_t           w[BW > 0 ? BW : 1];
 #pragma unroll
-	for (uint32_t r = 0; r < static_cast<uint32_t>(B); ++r) {
-		// the second word row is read unconditionally, clamped inside the vector
-		const uint32_t o = r * bw, k = o / B, s = o % B;
-		const uint32_t lo_word = __ldg(src + 32u * k + t);
-		const uint32_t hi_word = __ldg(src + 32u * min(k + 1u, last) + t);
-		const uint32_t hi      = (hi_word << (B - s)) & (((N::kLow << (B - s)) & N::kLow) * N::kRep);
-		const uint32_t x       = (((lo_word >> s) & ((N::kLow >> s) * N::kRep)) |
-		                    (s + bw > static_cast<uint32_t>(B) ? hi : 0u)) & vm;
+	for (int k = 0; k < BW; ++k) { w[k] = __ldg(src + 32 * k + t); }
+	uint32_t ev = 0, od = 0;
+#pragma unroll
+	for (int r = 0; r < B; ++r) {
+		const int o = r * BW, k = o / B, sh = o % B;
+		uint32_t  x = 0;
+		if constexpr (BW > 0) {
+			x = (w[k] >> sh) & ((N::kLow >> sh & V) * N::kRep);
+			if (sh + BW > B) { x |= (w[k + 1] << (B - sh)) & ((N::kLow << (B - sh) & V) * N::kRep); }
+		}
+		uint32_t y = x;
 		if constexpr (NOWRAP) {
-			// at most 8 (B = 8) or 16 (B = 16) rows of B-bit fields per half
+			y = x + base_rep;
+		} else {
+			y = ((x & ~N::kHigh) + (base_rep & ~N::kHigh)) ^ ((x ^ base_rep) & N::kHigh);
+		}
+		if constexpr (OUT) { __stcs(dst + 32 * r + t, y); }
+		if constexpr (kFields && kPacked) {
+			ev += x;
+		} else if constexpr (kFields) {
 			if constexpr (B == 8) {
 				ev += x & 0x00ff00ffu;
 				od += (x >> 8) & 0x00ff00ffu;
@@ -76,11 +106,7 @@ __device__ __forceinline__ void narrow_vector(const uint32_t* __restrict src, ui
 				ev += x & 0xffffu;
 				od += x >> 16;
 			}
-			continue;
-		}
-		const uint32_t y = ((x & ~N::kHigh) + (base_rep & ~N::kHigh)) ^ ((x ^ base_rep) & N::kHigh);
-		if constexpr (OUT) { __stcs(dst + 32u * r + t, y); }
-		if constexpr (SUM) {
+		} else if constexpr (SUM) {
 			uint32_t keep = y;
 			if constexpr (TAIL) {
 				keep = 0;
@@ -92,8 +118,10 @@ __device__ __forceinline__ void narrow_vector(const uint32_t* __restrict src, ui
 			part += lane_sum<B>(keep);
 		}
 	}
-	if constexpr (NOWRAP) {
-		if constexpr (B == 8) {
+	if constexpr (kFields) {
+		if constexpr (kPacked) {
+			part += lane_sum<B>(ev);
+		} else if constexpr (B == 8) {
 			part += (ev & 0xffffu) + (ev >> 16) + (od & 0xffffu) + (od >> 16);
 		} else {
 			part += ev + od;
@@ -103,58 +131,81 @@ __device__ __forceinline__ void narrow_vector(const uint32_t* __restrict src, ui
 }
 
 // Resident 256-thread blocks per SM asked of the compiler (it trades
-// registers for warps), measured per form on B200 at 2^28 values: decode to
-// HBM 4, 8-bit sums and 64-bit lanes 3, 16-bit sums 2.
-template <int B, bool OUT, bool SUM>
-constexpr int narrow_min_blocks() {
-	return OUT && !SUM ? 4 : (B == 16 && !OUT ? 2 : 3);
-}
+// registers for warps): enough warps to cover the reads, and registers for
+// two vectors' words.
+constexpr int kNarrowMinBlocks = 4;
 
-// 8/16-bit lanes: one warp per vector (a 0-bit column reads no payload).
-template <int B, bool OUT, bool SUM>
-__global__ void __launch_bounds__(256, narrow_min_blocks<B, OUT, SUM>()) decode_narrow_kernel(const uint32_t* __restrict in, uint64_t n, uint64_t n_vec,
-                                                            uint32_t bw, uint32_t base_rep, uint32_t* __restrict out,
-                                                            unsigned long long* sum, bool nowrap) {
-	using N                = Narrow<B>;
-	const uint32_t     t   = threadIdx.x & 31u;
-	const uint64_t     wg  = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-	const uint64_t     nw  = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-	const uint32_t     vm  = (bw >= static_cast<uint32_t>(B) ? N::kLow : (1u << bw) - 1u) * N::kRep;
-	unsigned long long acc = 0;
-	for (uint64_t v = wg; v < n_vec; v += nw) {
-		const uint32_t* src  = in + v * 32u * bw;
-		uint32_t*       dst  = OUT ? out + v * 32u * B : nullptr;
-		const uint64_t  rem  = n - v * 1024u;
+// A column of width BW: one warp per vector.
+template <int B, int BW, bool OUT, bool SUM, bool NOWRAP>
+__device__ __forceinline__ void narrow_column(const uint32_t* __restrict in, uint64_t n, uint64_t n_vec,
+                                              uint32_t base_rep, uint32_t* __restrict out, unsigned long long& acc) {
+	const uint32_t t  = threadIdx.x & 31u;
+	const uint64_t wg = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+	const uint64_t nw = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+	const uint64_t full = SUM ? n / 1024u : n_vec; // vectors that need no test of their rows
+	uint64_t       v    = wg;
+	// Several vectors at a time while their words are few, so that enough
+	// reads are in flight (sum of 90 M 8-bit values at width 3, whole call: 22.2
+	// us one by one, 20.5 four at a time).
+	constexpr uint32_t U = BW <= 4 ? 4u : BW <= 8 ? 2u : 1u;
+	for (; U > 1u && v + (U - 1u) * nw < full; v += U * nw) {
+#pragma unroll
+		for (uint32_t u = 0; u < U; ++u) {
+			uint32_t part = 0;
+			narrow_vector<B, BW, OUT, SUM, false, NOWRAP>(in + (v + u * nw) * (32u * BW),
+			                                              OUT ? out + (v + u * nw) * (32u * B) : nullptr, base_rep, t,
+			                                              1024u, part);
+			acc += part;
+		}
+	}
+	for (; v < n_vec; v += nw) {
+		const uint32_t* src  = in + v * (32u * BW);
+		uint32_t*       dst  = OUT ? out + v * (32u * B) : nullptr;
 		uint32_t        part = 0;
-		if (bw == 0) {
-			// every value is the base
-			for (uint32_t r = 0; r < static_cast<uint32_t>(B); ++r) {
-				if constexpr (OUT) { __stcs(dst + 32u * r + t, base_rep); }
-			}
-			if constexpr (SUM) {
-				const uint64_t cnt = rem < 1024u ? rem : 1024u;
-				if (t == 0) { acc += cnt * (base_rep & N::kLow); }
-			}
-		} else if (rem >= 1024u) {
-			if constexpr (SUM && !OUT) {
-				if (nowrap) {
-					narrow_vector<B, OUT, SUM, false, true>(src, dst, bw, vm, base_rep, t, rem, part);
-				} else {
-					narrow_vector<B, OUT, SUM, false>(src, dst, bw, vm, base_rep, t, rem, part);
-				}
-			} else {
-				narrow_vector<B, OUT, SUM, false>(src, dst, bw, vm, base_rep, t, rem, part);
-			}
+		if (v < full) {
+			narrow_vector<B, BW, OUT, SUM, false, NOWRAP>(src, dst, base_rep, t, 1024u, part);
 		} else {
-			narrow_vector<B, OUT, SUM, true>(src, dst, bw, vm, base_rep, t, rem, part);
+			narrow_vector<B, BW, OUT, SUM, true, NOWRAP>(src, dst, base_rep, t, n - v * 1024u, part);
 		}
 		acc += part;
 	}
-	if constexpr (SUM) {
-#pragma unroll
-		for (int off = 16; off > 0; off >>= 1) { acc += __shfl_xor_sync(0xffffffffu, acc, off); }
-		if (t == 0 && acc) { atomicAdd(sum, acc); }
+}
+
+// 8/16-bit lanes: one warp per vector (a 0-bit column reads no payload); the
+// width is a switch ahead of the loop over the vectors.
+template <int B, bool OUT, bool SUM, bool NOWRAP>
+__global__ void __launch_bounds__(256, kNarrowMinBlocks) decode_narrow_kernel(const uint32_t* __restrict in, uint64_t n,
+                                                                             uint64_t n_vec, uint32_t bw,
+                                                                             uint32_t base_rep,
+                                                                             uint32_t* __restrict out,
+                                                                             unsigned long long* sum) {
+	unsigned long long acc = 0;
+	switch (bw) {
+#define FLS_NARROW_CASE(W)                                                                                             \
+	case W:                                                                                                            \
+		if constexpr (W <= B) { narrow_column<B, W, OUT, SUM, NOWRAP>(in, n, n_vec, base_rep, out, acc); }             \
+		break;
+		FLS_NARROW_CASE(0)
+		FLS_NARROW_CASE(1)
+		FLS_NARROW_CASE(2)
+		FLS_NARROW_CASE(3)
+		FLS_NARROW_CASE(4)
+		FLS_NARROW_CASE(5)
+		FLS_NARROW_CASE(6)
+		FLS_NARROW_CASE(7)
+		FLS_NARROW_CASE(8)
+		FLS_NARROW_CASE(9)
+		FLS_NARROW_CASE(10)
+		FLS_NARROW_CASE(11)
+		FLS_NARROW_CASE(12)
+		FLS_NARROW_CASE(13)
+		FLS_NARROW_CASE(14)
+		FLS_NARROW_CASE(15)
+		FLS_NARROW_CASE(16)
+#undef FLS_NARROW_CASE
+	default: break;
 	}
+	if constexpr (SUM) { add_block_sum(acc, sum); }
 }
 
 // 64-bit lanes: a half-warp per vector, one lane per thread.
@@ -215,8 +266,7 @@ __global__ void __launch_bounds__(256, 3) decode_u64_kernel(const uint64_t* __re
 		}
 	}
 	if constexpr (SUM) {
-#pragma unroll
-		for (int off = 16; off > 0; off >>= 1) { acc += __shfl_xor_sync(0xffffffffu, acc, off); }
+		acc = warp_sum_u64(acc);
 		if ((threadIdx.x & 31u) == 0 && acc) { atomicAdd(sum, acc); }
 	}
 }
@@ -265,13 +315,16 @@ fls_status launch_decode(uint32_t bits, const void* d_in, uint64_t n, uint8_t bw
 		const bool nowrap = (base & ((1ull << bits) - 1u)) + ((1ull << bw) - 1u) < (1ull << bits);
 		const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>((n_vec + 7u) / 8u, static_cast<uint64_t>(di.sms) * 16u));
 		launch_mode(d_out != nullptr, d_sum != nullptr, [&](auto mode) {
-			constexpr int M = decltype(mode)::value;
+			constexpr int  M   = decltype(mode)::value;
+			constexpr bool O = (M & 1) != 0, S = (M & 2) != 0;
+			const auto     run = [&](auto* kernel) {
+                kernel<<<grid, 256, 0, st>>>(static_cast<const uint32_t*>(d_in), n, n_vec, bw, rep,
+                                             static_cast<uint32_t*>(d_out), sum);
+			};
 			if (bits == 8) {
-				decode_narrow_kernel<8, (M & 1) != 0, (M & 2) != 0><<<grid, 256, 0, st>>>(
-				    static_cast<const uint32_t*>(d_in), n, n_vec, bw, rep, static_cast<uint32_t*>(d_out), sum, nowrap);
+				nowrap ? run(decode_narrow_kernel<8, O, S, true>) : run(decode_narrow_kernel<8, O, S, false>);
 			} else {
-				decode_narrow_kernel<16, (M & 1) != 0, (M & 2) != 0><<<grid, 256, 0, st>>>(
-				    static_cast<const uint32_t*>(d_in), n, n_vec, bw, rep, static_cast<uint32_t*>(d_out), sum, nowrap);
+				nowrap ? run(decode_narrow_kernel<16, O, S, true>) : run(decode_narrow_kernel<16, O, S, false>);
 			}
 		});
 	}

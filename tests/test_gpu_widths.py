@@ -74,3 +74,20 @@ def test_sum_only_every_bit_width(cuda, bits, dt):
             v = _column(g, dt, bits, bw, n, base)
             _, total = _run(v, dt, bits, bw, base, want_out=False)
             assert total == int(v.astype(np.uint64).sum(dtype=np.uint64)), (bw, base)
+
+
+@pytest.mark.parametrize("bits,dt", WIDTHS[:2])
+@pytest.mark.parametrize("n", [1, 1024, 4 * 1024 + 1023])
+def test_narrow_widths_at_the_wrap(cuda, bits, dt, n):
+    """Every width of the narrow lanes with bases just below and at the one that
+    makes the largest value wrap; largest fields only, so packed sums are at
+    their bound; decode and sum alone and together."""
+    for bw in range(bits + 1):
+        for base in sorted({0, (1 << bits) - (1 << bw), min((1 << bits) - (1 << bw) + 1, (1 << bits) - 1)}):
+            v = (np.full(n, (1 << bw) - 1, np.uint64) + np.uint64(base)).astype(dt)
+            for want_out, want_sum in ((True, False), (False, True), (True, True)):
+                out, total = _run(v, dt, bits, bw, base, want_out, want_sum)
+                if want_out:
+                    assert np.array_equal(out.cpu().numpy().view(dt)[:n], v)
+                if want_sum:
+                    assert total == int(v.astype(np.uint64).sum())
