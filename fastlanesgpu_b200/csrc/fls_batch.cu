@@ -187,7 +187,34 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) batch_kernel(const __grid_c
 				uint32_t x[32];
 				dev::decode_vals(sf, vf, base + L.dict, lane, x);
 				long long p[kGroupQueries] = {0, 0, 0, 0};
-				if (same && valid == 0xffffffffu) {
+				// A value's distance from vbase (the FOR or dictionary base, or
+				// a DELTA lane's first value) is below 2^21 when `narrow`, and
+				// vbase plus it does not wrap an int32.
+				const uint32_t vbase  = vf.scheme == FLS_SCHEME_DELTA ? sf[lane] : static_cast<uint32_t>(vf.base);
+				const uint32_t widest = vf.scheme == FLS_SCHEME_DELTA ? 16u : vf.scheme == FLS_SCHEME_CONST ? 32u : 21u;
+				const bool     narrow = same && valid == 0xffffffffu && vf.bw <= widest &&
+				                    static_cast<int32_t>(vbase) <= INT32_MAX - (1 << 21);
+				if (__all_sync(0xffffffffu, narrow)) {
+					// Sum and count of a query share a word: distances of 32 rows
+					// below 2^26, their number above it (3 instructions per value
+					// and query, 6 with a 64-bit sum; 24 columns, 96 queries: kernel
+					// 58 -> 49 us).
+					uint32_t w[kGroupQueries] = {0, 0, 0, 0};
+					const uint32_t up = (1u << 26) - vbase;
+#pragma unroll
+					for (int r = 0; r < 32; ++r) {
+						const uint32_t y = x[r] + up;
+#pragma unroll
+						for (uint32_t j = 0; j < kGroupQueries; ++j) { w[j] += x[r] - lo[j] <= range[j] ? y : 0u; }
+					}
+#pragma unroll
+					for (uint32_t j = 0; j < kGroupQueries; ++j) {
+						const uint32_t c = live[j] ? w[j] >> 26 : 0u, d = live[j] ? w[j] & ((1u << 26) - 1u) : 0u;
+						cnt[j] += c;
+						p[j] = static_cast<long long>(d) +
+						       static_cast<long long>(static_cast<int32_t>(vbase)) * static_cast<long long>(c);
+					}
+				} else if (same && valid == 0xffffffffu) {
 					// A whole vector whose sums are over the filtered values: each
 					// query adds the rows in its range straight from the registers.
 #pragma unroll

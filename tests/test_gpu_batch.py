@@ -151,3 +151,23 @@ def test_batch_pieces_of_uneven_items(cuda, chunk, lens):
             assert tuple(got[i]) == _want(vals, q)
     ops.check_device_error()
     b.close()
+
+
+@pytest.mark.parametrize("bits", [16, 17, 21, 22, 31])
+@pytest.mark.parametrize("top", [False, True])
+def test_batch_sums_at_the_word_bound(cuda, bits, top):
+    """Vectors whose distances from the base just fit, or do not fit, the shared
+    sum-and-count word: every row at the largest distance and selected, bases at
+    the top and the bottom of int32, every scheme."""
+    base = 2**31 - 2**bits if top else -(2**31)
+    flat = np.full(1024, base + 2**bits - 1, np.int64)
+    flat[:32] = base
+    v = np.concatenate([flat, np.full(1024, base), flat[::-1]]).astype(np.int32)
+    ramp = np.sort(np.resize(np.linspace(base, base + 2**bits - 1, 97).astype(np.int64), 1024)).astype(np.int32)
+    v = np.concatenate([v, ramp, v[:1000]])
+    cols = [EncodedColumn.encode(v, s).to_device() for s in (0, 1, 2, 3, 4)]
+    qs = [(c, lo, hi, c) for c in range(5) for lo, hi in ((-2**31, 2**31 - 1), (int(v[40]), 2**31 - 1), (base, base), (5, 4))]
+    got = Batch(cols, qs).run().cpu().numpy()
+    for i, q in enumerate(qs):
+        assert tuple(got[i]) == _want([v] * 5, q)
+    ops.check_device_error()
