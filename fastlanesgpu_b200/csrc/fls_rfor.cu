@@ -8,15 +8,23 @@
 // the lengths into run ends, the ends are marked in shared memory, a second
 // block scan turns the marks into each position's run index, and the values
 // are gathered.  Here one warp decodes a tile with no block-wide barrier:
-//   1. lane l unpacks a contiguous chunk of the runs' lengths, and one warp
-//      scan of the chunk sums gives each run's first position;
-//   2. each lane writes its runs' values to shared memory and sets the bit of
-//      each run's first position in a 512-bit mask (16 words);
-//   3. position p = 32 j + l (row j of the tile as 32 coalesced words) is in
-//      run popc(mask bits 0..p) - 1: one broadcast word, one popc and a prefix
-//      count per row; the value is gathered from shared memory.
+//   1. lane l takes runs l, l + 32, ...: 32 fields of a packed block fill
+//      exactly bw words, so a lane's fields all start at the same bit and its
+//      shift and mask are constants; a warp scan of the lengths per 32 runs
+//      gives each run's first position;
+//   2. the sum needs no more: a run adds its value times its length;
+//   3. to memory, each lane writes its runs' values to shared memory and sets
+//      the bit of each run's first position in a 512-bit mask (16 words);
+//   4. a lane writes four consecutive positions at a time: the first is in run
+//      popc(mask bits up to it) - 1, each next one a run further where its bit
+//      is set; the values are gathered from shared memory.
 // A tile whose block is inconsistent is skipped and flagged, never read past
 // its stream.
+//
+// Bounded by integer issue (70 % of it active).  16.8 M values of geometric
+// runs (mean 16), kernel, against contiguous chunks of runs per lane, one
+// position per lane and row and the sum over expanded positions: to memory
+// 20.7 -> 19.3 us, sum 20.5 -> 13.1.
 #include "fls_pipeline.cuh"
 
 namespace fls {
@@ -38,136 +46,179 @@ __device__ __forceinline__ uint32_t packed_words(uint32_t count, uint32_t bw) {
 	return bits == 0 ? 1u : (bits + 31u) >> 5;
 }
 
-// Field k of a sequentially packed block (bit k*bw, LSB first); never reads
-// past the block's last packed word.
-__device__ __forceinline__ uint32_t field(const uint32_t* __restrict__ p, uint32_t k, uint32_t bw) {
-	if (bw == 0) { return 0u; }
-	const uint32_t bit = k * bw, w = bit >> 5, sh = bit & 31u;
-	const uint32_t lo  = __ldg(p + w);
-	const uint32_t hi  = (sh + bw > 32u) ? __ldg(p + w + 1) : 0u;
-	const uint32_t m   = bw >= 32 ? 0xffffffffu : ((1u << bw) - 1u);
-	return __funnelshift_r(lo, hi, sh) & m;
-}
+// A lane's fields lane, lane + 32, ... of a sequentially packed block (bit
+// k*bw, LSB first): word row i of bw words holds fields 32 i .. 32 i + 31.
+// Never reads past the block's last packed word.
+struct LaneFields {
+	const uint32_t* p;
+	uint32_t        bw, sh, mask, next;
+	__device__ __forceinline__ LaneFields(const uint32_t* block, uint32_t width, uint32_t lane) {
+		const uint32_t bit = lane * width;
+		p    = block + (bit >> 5);
+		bw   = width;
+		sh   = bit & 31u;
+		mask = width >= 32 ? 0xffffffffu : ((1u << width) - 1u);
+		next = sh + width > 32u ? 1u : 0u; // without a second word the first is read twice and masked off
+	}
+	// Row i's field; the caller has checked that it is one of the block's.
+	__device__ __forceinline__ uint32_t get(uint32_t i) const {
+		if (bw == 0) { return 0u; } // warp-uniform
+		const uint32_t* q = p + i * bw;
+		return __funnelshift_r(__ldg(q), __ldg(q + next), sh) & mask;
+	}
+};
 
-// The run index and value of position 32 j + lane for the 16 rows of a tile,
-// handed to f(p, v); pre = run starts before mask word `lane`, minus one.
-template <bool FULL, class F>
-__device__ __forceinline__ void expand_rows(const uint32_t* bits, const uint32_t* vals, uint32_t pre, uint32_t lane,
-                                            uint32_t live, F&& f) {
-	const uint32_t upto = 0xffffffffu >> (31u - lane);
+// The values of a tile's positions, four consecutive ones at a time per lane
+// (positions 128 j + 4 lane .. + 3), handed to f(first position, values);
+// words[w] = {mask bits of positions 32 w .. 32 w + 31, run starts before them
+// minus one}.
+template <class F>
+__device__ __forceinline__ void expand_rows(const uint2* words, const uint32_t* vals, uint32_t lane, F&& f) {
+	const uint32_t sh = 4u * (lane & 7u), upto = 0xffffffffu >> (31u - sh);
 #pragma unroll
-	for (uint32_t j = 0; j < kTile / 32; ++j) {
-		const uint32_t w   = bits[j];
-		const uint32_t idx = __shfl_sync(0xffffffffu, pre, j) + __popc(w & upto);
-		const uint32_t p   = 32u * j + lane;
-		if (FULL || p < live) { f(p, vals[idx]); }
+	for (uint32_t j = 0; j < kTile / 128; ++j) {
+		const uint2 w = words[4u * j + (lane >> 3)];
+		uint32_t    k = w.y + __popc(w.x & upto);
+		uint4       v;
+		v.x = vals[k];
+		k += (w.x >> (sh + 1u)) & 1u;
+		v.y = vals[k];
+		k += (w.x >> (sh + 2u)) & 1u;
+		v.z = vals[k];
+		k += (w.x >> (sh + 3u)) & 1u;
+		v.w = vals[k];
+		f(128u * j + 4u * lane, v);
 	}
 }
 
-template <bool SUM>
-__global__ void __launch_bounds__(kRforWarps * 32, 5) rfor_kernel(const __grid_constant__ RforParams P) {
-	__shared__ uint32_t s_vals[kRforWarps][kTile];
-	__shared__ uint16_t s_lens[kRforWarps][kTile];
-	__shared__ uint32_t s_bits[kRforWarps][kTile / 32];
+// A tile's two blocks {minimum, bit width per byte, count, fields}, read and
+// checked by one lane: 32 tiles of the warp at a time, so that a tile costs
+// five shuffles where every lane read and checked the same words, two round
+// trips to memory one after the other.
+constexpr uint32_t kBadTile = 0xffffffffu;
+struct TileHead {
+	uint32_t vo, ro;     // 32-bit word offsets of the blocks
+	uint32_t vmin, rmin;
+	uint32_t widths;     // count | value width << 16 | length width << 24, or kBadTile
+};
+
+__device__ __forceinline__ TileHead load_head(const RforParams& P, uint64_t t) {
+	TileHead h {0u, 0u, 0u, 0u, kBadTile};
+	if (t >= P.n_tiles) { return h; }
+	const uint32_t vo = __ldg(P.val_off + t), ve = __ldg(P.val_off + t + 1);
+	const uint32_t ro = __ldg(P.rl_off + t), re = __ldg(P.rl_off + t + 1);
+	bool           ok = static_cast<uint64_t>(vo) + 3u <= ve && ve <= P.n_val_words &&
+	          static_cast<uint64_t>(ro) + 3u <= re && re <= P.n_rl_words;
+	if (ok) {
+		const uint32_t *v = P.vals + vo, *r = P.rls + ro;
+		const uint32_t  vbw = __ldg(v + 1) & 0xffu, rbw = __ldg(r + 1) & 0xffu, cnt = __ldg(v + 2);
+		h.vmin = __ldg(v);
+		h.rmin = __ldg(r);
+		ok     = vbw <= 32u && rbw <= 32u && cnt >= 1u && cnt <= kTile && __ldg(r + 2) == cnt &&
+		     static_cast<uint64_t>(vo) + 3u + packed_words(cnt, vbw) <= ve &&
+		     static_cast<uint64_t>(ro) + 3u + packed_words(cnt, rbw) <= re;
+		h.vo     = vo;
+		h.ro     = ro;
+		h.widths = ok ? cnt | (vbw << 16) | (rbw << 24) : kBadTile;
+	}
+	if (!ok) { raise_err(P.err, kErrBadMeta); }
+	return h;
+}
+
+// WIDE: the output is 16-byte aligned.
+template <bool SUM, bool WIDE>
+__global__ void __launch_bounds__(kRforWarps * 32, 6) rfor_kernel(const __grid_constant__ RforParams P) {
+	__shared__ uint32_t s_vals[SUM ? 1 : kRforWarps][kTile];
+	__shared__ uint2    s_words[SUM ? 1 : kRforWarps][kTile / 32];
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	uint32_t*      vals = s_vals[warp];
-	uint16_t*      lens = s_lens[warp];
-	uint32_t*      bits = s_bits[warp];
+	uint32_t*      vals  = s_vals[SUM ? 0 : warp];
+	uint2*         words = s_words[SUM ? 0 : warp];
 	unsigned long long acc = 0;
-	const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kRforWarps;
-	uint64_t       t      = static_cast<uint64_t>(blockIdx.x) * kRforWarps + warp;
-	// block extents of the next tile, loaded one tile ahead
-	uint32_t nvo = 0, nve = 0, nro = 0, nre = 0;
-	if (t < P.n_tiles) {
-		nvo = __ldg(P.val_off + t);
-		nve = __ldg(P.val_off + t + 1);
-		nro = __ldg(P.rl_off + t);
-		nre = __ldg(P.rl_off + t + 1);
-	}
-	for (; t < P.n_tiles; t += stride) {
-		// the tile's blocks: {minimum, bit width per byte, count, fields}
-		const uint64_t vo = nvo, ve = nve, ro = nro, re = nre; // 32-bit word offsets
-		if (t + stride < P.n_tiles) {
-			nvo = __ldg(P.val_off + t + stride);
-			nve = __ldg(P.val_off + t + stride + 1);
-			nro = __ldg(P.rl_off + t + stride);
-			nre = __ldg(P.rl_off + t + stride + 1);
+	const uint64_t total = static_cast<uint64_t>(gridDim.x) * kRforWarps;
+	const uint64_t first = static_cast<uint64_t>(blockIdx.x) * kRforWarps + warp;
+	TileHead       head {};
+	uint32_t       j = 31u; // lane that holds the current tile
+	for (uint64_t t = first; t < P.n_tiles; t += total) {
+		j = (j + 1u) & 31u;
+		if (j == 0) { head = load_head(P, t + lane * total); }
+		const uint32_t widths = __shfl_sync(0xffffffffu, head.widths, j);
+		if (widths == kBadTile) { continue; } // flagged by the lane that read it
+		const uint32_t cnt  = widths & 0xffffu;
+		const uint32_t vmin = __shfl_sync(0xffffffffu, head.vmin, j), rmin = __shfl_sync(0xffffffffu, head.rmin, j);
+		const LaneFields vf(P.vals + __shfl_sync(0xffffffffu, head.vo, j) + 3u, (widths >> 16) & 0xffu, lane);
+		const LaneFields rf(P.rls + __shfl_sync(0xffffffffu, head.ro, j) + 3u, widths >> 24, lane);
+		const uint64_t   row0 = t * kTile;
+		const uint32_t   live = static_cast<uint32_t>(min(static_cast<uint64_t>(kTile), P.n_values - row0));
+		if constexpr (!SUM) {
+			if (lane < kTile / 32) { words[lane] = make_uint2(0u, 0u); }
+			__syncwarp();
 		}
-		bool     ok = vo + 3u <= ve && ve <= P.n_val_words && ro + 3u <= re && re <= P.n_rl_words;
-		uint32_t vmin = 0, vbw = 0, cnt = 0, rmin = 0, rbw = 0;
-		if (ok) {
-			vmin = __ldg(P.vals + vo);
-			vbw  = __ldg(P.vals + vo + 1) & 0xffu;
-			cnt  = __ldg(P.vals + vo + 2);
-			rmin = __ldg(P.rls + ro);
-			rbw  = __ldg(P.rls + ro + 1) & 0xffu;
-			ok   = vbw <= 32u && rbw <= 32u && cnt >= 1u && cnt <= kTile && __ldg(P.rls + ro + 2) == cnt &&
-			     vo + 3u + packed_words(cnt, vbw) <= ve && ro + 3u + packed_words(cnt, rbw) <= re;
+		// Runs 32 i + lane, until the tile's runs are used up (a tile whose
+		// runs do not cover it exactly is found out at the end: nothing of it
+		// has been added or written by then).
+		uint32_t           start = 0; // of the next 32 runs
+		unsigned long long part  = 0;
+		bool               fits  = true;
+		for (uint32_t i = 0; 32u * i < cnt; ++i) {
+			const uint32_t k    = 32u * i + lane;
+			const bool     mine = k < cnt;
+			uint32_t       l = 0, v = 0;
+			if (mine) {
+				l = rmin + rf.get(i);
+				v = vmin + vf.get(i);
+			}
+			fits          = fits && l <= kTile; // sums of 32 lengths below stay far from 32 bits
+			uint32_t incl = l;
+#pragma unroll
+			for (int o = 1; o < 32; o <<= 1) {
+				const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+				if (lane >= static_cast<uint32_t>(o)) { incl += x; }
+			}
+			const uint32_t pos = start + incl - l;
+			if constexpr (SUM) {
+				// the run's positions below `live`
+				part += static_cast<unsigned long long>(v) * (min(pos + l, live) - min(pos, live));
+			} else if (mine) {
+				vals[k] = v;
+				if (pos < kTile) { atomicOr(&words[pos >> 5].x, 1u << (pos & 31u)); } // a run of length 0 may end the tile
+			}
+			start += __shfl_sync(0xffffffffu, incl, 31);
+			if (!__all_sync(0xffffffffu, fits)) { break; }
 		}
-		if (!ok) { // warp-uniform: every lane read the same words
+		if (start != kTile || !__all_sync(0xffffffffu, fits)) { // the runs must cover the tile exactly
 			if (lane == 0) { raise_err(P.err, kErrBadMeta); }
+			__syncwarp();
 			continue;
 		}
-		const uint32_t* vf = P.vals + vo + 3u;
-		const uint32_t* rf = P.rls + ro + 3u;
-		// 1. this lane's chunk of runs: values and lengths to shared memory,
-		//    and where the chunk starts
-		const uint32_t chunk = (cnt + 31u) >> 5;
-		const uint32_t k0 = min(cnt, lane * chunk), k1 = min(cnt, k0 + chunk);
-		uint32_t       len = 0;
-		for (uint32_t k = k0; k < k1; ++k) {
-			const uint32_t l = rmin + field(rf, k, rbw);
-			vals[k] = vmin + field(vf, k, vbw);
-			lens[k] = static_cast<uint16_t>(min(l, kTile)); // a longer run fails the cover check below
-			len += l;
-		}
-		uint32_t incl = len;
-#pragma unroll
-		for (int o = 1; o < 32; o <<= 1) {
-			const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-			if (lane >= static_cast<uint32_t>(o)) { incl += x; }
-		}
-		if (__shfl_sync(0xffffffffu, incl, 31) != kTile) { // the runs must cover the tile exactly
-			if (lane == 0) { raise_err(P.err, kErrBadMeta); }
-			continue;
-		}
-		// 2. run starts into the mask (each lane reads back its own lengths)
-		if (lane < kTile / 32) { bits[lane] = 0u; }
-		__syncwarp();
-		uint32_t pos = incl - len;
-		for (uint32_t k = k0; k < k1; ++k) {
-			if (pos < kTile) { atomicOr(&bits[pos >> 5], 1u << (pos & 31u)); } // runs of length 0 end at the tile's end
-			pos += lens[k];
-		}
-		__syncwarp();
-		// 3. run index of position 32 j + lane from prefix counts of the mask words
-		const uint32_t own = lane < kTile / 32 ? __popc(bits[lane]) : 0u;
-		uint32_t       c   = own;
-#pragma unroll
-		for (int o = 1; o < 16; o <<= 1) {
-			const uint32_t x = __shfl_up_sync(0xffffffffu, c, o);
-			if (lane >= static_cast<uint32_t>(o)) { c += x; }
-		}
-		const uint32_t pre  = c - own - 1u; // starts before word lane, minus one
-		const uint64_t row0 = t * kTile;
-		const uint32_t live = static_cast<uint32_t>(min(static_cast<uint64_t>(kTile), P.n_values - row0));
 		if constexpr (SUM) {
-			auto add = [&](uint32_t, uint32_t v) { acc += v; };
-			if (live == kTile) {
-				expand_rows<true>(bits, vals, pre, lane, live, add);
-			} else {
-				expand_rows<false>(bits, vals, pre, lane, live, add);
-			}
+			acc += part;
 		} else {
-			uint32_t* out = P.out + row0;
-			auto      put = [&](uint32_t p, uint32_t v) { __stcs(out + p, v); };
-			if (live == kTile) {
-				expand_rows<true>(bits, vals, pre, lane, live, put);
-			} else {
-				expand_rows<false>(bits, vals, pre, lane, live, put);
+			__syncwarp();
+			// run starts before each mask word, minus one
+			const uint32_t own = lane < kTile / 32 ? __popc(words[lane].x) : 0u;
+			uint32_t       c   = own;
+#pragma unroll
+			for (int o = 1; o < 16; o <<= 1) {
+				const uint32_t x = __shfl_up_sync(0xffffffffu, c, o);
+				if (lane >= static_cast<uint32_t>(o)) { c += x; }
 			}
+			if (lane < kTile / 32) { words[lane].y = c - own - 1u; }
+			__syncwarp();
+			uint32_t* out = P.out + row0;
+			if (WIDE && live == kTile) {
+				expand_rows(words, vals, lane,
+				            [&](uint32_t p, const uint4& v) { __stcs(reinterpret_cast<uint4*>(out + p), v); });
+			} else {
+				expand_rows(words, vals, lane, [&](uint32_t p, const uint4& v) {
+					const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+					for (uint32_t i = 0; i < 4; ++i) {
+						if (p + i < live) { __stcs(out + p + i, e[i]); }
+					}
+				});
+			}
+			__syncwarp();
 		}
-		__syncwarp();
 	}
 	if constexpr (SUM) {
 		const unsigned long long s = warp_sum_u64(acc);
@@ -203,11 +254,13 @@ fls_status rfor_launch(const fls_rfor_column* col, uint32_t* d_out, uint64_t* d_
 		return s;
 	}
 	const uint32_t grid = static_cast<uint32_t>(
-	    std::min<uint64_t>((P.n_tiles + kRforWarps - 1) / kRforWarps, static_cast<uint64_t>(di.sms) * 8u));
+	    std::min<uint64_t>((P.n_tiles + kRforWarps - 1) / kRforWarps, static_cast<uint64_t>(di.sms) * 6u)); // resident
 	if (d_sum) {
-		rfor_kernel<true><<<grid, kRforWarps * 32, 0, st>>>(P);
+		rfor_kernel<true, false><<<grid, kRforWarps * 32, 0, st>>>(P);
+	} else if ((reinterpret_cast<uintptr_t>(d_out) & 15u) == 0) {
+		rfor_kernel<false, true><<<grid, kRforWarps * 32, 0, st>>>(P);
 	} else {
-		rfor_kernel<false><<<grid, kRforWarps * 32, 0, st>>>(P);
+		rfor_kernel<false, false><<<grid, kRforWarps * 32, 0, st>>>(P);
 	}
 	count_launch();
 	return cuda_check(cudaGetLastError(), "rfor_kernel launch");

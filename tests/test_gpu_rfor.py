@@ -125,3 +125,21 @@ def test_decode_time_against_reference_gpu_decoder(cuda):
         assert torch.equal(out.cpu(), torch.from_numpy(vals)), name
     print("\nRFOR decode of 2^26 values to HBM, ms per launch:",
           ", ".join(f"{k} {v:.4f}" for k, v in ms.items()))
+
+
+@pytest.mark.parametrize("n", [1, 511, 512, 513, 512 * 40 + 3])
+@pytest.mark.parametrize("mean_run", [1.0, 1.02, 8.0, 600.0])
+def test_rfor_rows_and_alignment(cuda, n, mean_run):
+    """From one run per value (16 groups of 32 runs) to one run per tile, into
+    16-byte aligned outputs and into ones that are not."""
+    import torch
+    vals = datagen.geometric_runs(n, mean_run=mean_run, value_bits=30, seed=n).astype(np.int32)
+    col = RforColumn.encode(vals).to_device()
+    for shift in (0, 1, 3):
+        buf = torch.full((n + shift + 4,), -1, dtype=torch.int32, device="cuda")
+        ops.rfor_decode(col, out=buf[shift:shift + n])
+        got = buf.cpu().numpy()
+        assert np.array_equal(got[shift:shift + n], vals)
+        assert np.all(got[:shift] == -1) and np.all(got[shift + n:] == -1)
+    assert int(ops.rfor_decode_sum(col).cpu()[0]) == int(vals.view(np.uint32).astype(np.uint64).sum())
+    ops.check_device_error()
