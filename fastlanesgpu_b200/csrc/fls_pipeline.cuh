@@ -308,6 +308,7 @@ int        tuning_group_smem();
 int        tuning_late_measure();
 int        tuning_half_vectors();
 uint32_t   tuning_table_words(); // table budget in 4-byte words
+uint32_t   launch_warps(uint32_t otherwise); // warps per CTA the caller set (fls_set_launch_config), if any
 uint32_t   jit_max_warps(); // most warps per CTA of the specialised join kernels
 
 // Validates one column descriptor and converts it for a kernel.

@@ -58,10 +58,12 @@ __global__ void err_take_kernel(uint32_t* words) { words[1] = atomicExch(&words[
 
 void count_launch(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-uint32_t jit_max_warps() {
+uint32_t launch_warps(uint32_t otherwise) {
 	std::lock_guard<std::mutex> lk(g_cfg_mu);
-	return g_warps_set ? g_cfg.warps : kJitDefaultWarps;
+	return g_warps_set ? g_cfg.warps : otherwise;
 }
+
+uint32_t jit_max_warps() { return launch_warps(kJitDefaultWarps); }
 
 namespace {
 constexpr int    kDefaultSparseRows = 4;
