@@ -150,10 +150,11 @@ __global__ void __launch_bounds__(Op::kWarps * 32, 1)
 // Lays out and launches: as many warps as the operator takes and shared
 // memory holds at two slots or more, then slots up to the launch
 // configuration's bytes in flight per warp (stages x tile bytes), or a third
-// of them where every vector is also written out: past that the reads in
-// flight only disturb the writes (50 M values to memory, FOR of mixed widths:
-// 49.7 us at 4 KB a warp, 52.3 at 12 KB; DELTA 45.0 and 46.5).  A column of
-// fewer vectors than warps spreads over the SMs.
+// of them where every vector is also written out (half in original order):
+// past that the reads in flight only disturb the writes (67 M values to
+// memory: DELTA 59.0 us at 4 KB a warp, 61.7 at 6 KB; in original order 59.4
+// at 6 KB, 59.8 at 4 and 61.0 at 8; FOR of mixed widths 68.5, 69.3 at 12).  A
+// column of fewer vectors than warps spreads over the SMs.
 template <class Op>
 fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_words, cudaStream_t stream) {
 	ColumnCfg  cfg {};
@@ -169,7 +170,7 @@ fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_wor
 	cfg.n_vec    = (col.n_values + 1023u) / 1024u;
 	const auto round4 = [](uint32_t w) { return (w + 3u) & ~3u; };
 	cfg.slot_words    = round4(cfg.col.slot_words);
-	const uint32_t flight = stages * tile_bytes / Op::kFlightShare;
+	const uint32_t flight = stages * tile_bytes / op.flight_share();
 	const uint32_t want   = std::max<uint32_t>(1u, flight / std::max<uint32_t>(4u * cfg.slot_words, 256u));
 	const uint32_t fixed = kSlotSlackWords + (cfg.has_dict ? kDictWords : 0u) + round4(extra_words) + 2u * kMaxSlots;
 	const uint32_t avail = static_cast<uint32_t>(di.max_smem) / 4u;
@@ -216,7 +217,8 @@ struct NoState {};
 // padded shared-memory tile (33 words per chunk, conflict-free) into original
 // order.
 struct DecodeOp {
-	static constexpr uint32_t kWarps = 16, kFlightShare = 3;
+	static constexpr uint32_t kWarps = 16;
+	uint32_t flight_share() const { return original ? 2u : 3u; }
 	using State = NoState;
 	uint32_t* out;
 	uint32_t  original;
@@ -248,7 +250,8 @@ struct AccState {
 // Decode fused with a uint64 sum; four independent partial sums per lane, one
 // atomic per warp at the end.
 struct DecodeSumOp {
-	static constexpr uint32_t kWarps = 16, kFlightShare = 1;
+	static constexpr uint32_t kWarps = 16;
+	uint32_t flight_share() const { return 1u; }
 	using State = AccState;
 	unsigned long long* sum;
 	__device__ void process(State& S, const ColumnVec& cv, uint32_t lane, const ColumnCfg& cfg) const {
@@ -400,7 +403,8 @@ template <uint32_t SCHEME>
 struct SchemeSumOp {
 	// 50 M values, kernel at 16, 24 and 32 warps (us): DELTA 20.2, 18.1, 18.4; RLE
 	// 29.7, 27.3, 26.5; DICT 43.5, 39.9, 39.9.
-	static constexpr uint32_t kWarps = 24, kFlightShare = 1;
+	static constexpr uint32_t kWarps = 24;
+	uint32_t flight_share() const { return 1u; }
 	using State = AccState;
 	unsigned long long* sum;
 	__device__ void process(State& S, const ColumnVec& sv, uint32_t lane, const ColumnCfg& cfg) const {
