@@ -128,7 +128,10 @@ __device__ void scan_tiles(const uint64_t* reports, uint64_t* offsets, uint64_t 
 		}
 		idle = pos == pos0 ? idle + 1u : 0u;
 		if (idle == kPollLimit) {
-			if (lane == 0) { atomicOr(err, kErrTimeout); }
+			if (lane == 0) {
+				atomicOr(err, kErrTimeout);
+				info[0] = info[1] = info[2] = 0;
+			}
 			for (uint64_t t = pos + lane; t < n_tiles; t += 32u) { tile_store(offsets + t, kTileLost); }
 			return;
 		}
