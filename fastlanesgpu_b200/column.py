@@ -263,28 +263,38 @@ class PendingEncode:
     encode_column_learned_gpu returns.  Deferring the read lets many columns
     be encoded back to back with no host round trip in between."""
 
-    def __init__(self, out, meta, info, schemes, n, layout, compact):
+    def __init__(self, out, meta, info, schemes, n, layout, compact, defer: bool = True):
         import torch
         self.out, self.meta, self.info, self.schemes = out, meta, info, schemes
         self.n, self.layout, self.compact = n, layout, compact
-        # The info words start on their way to the host right behind the
-        # encode, so finish() waits for this encode only and not for the ones
-        # enqueued after it.  (Not while capturing: finish() then reads them.)
-        self._host = self._done = None
-        if not torch.cuda.is_current_stream_capturing():
-            self._host = torch.empty(4, dtype=torch.int64, pin_memory=True)
-            self._host.copy_(info, non_blocking=True)
+        # finish() waits for this encode only, not for what is enqueued after
+        # it.  (Not while capturing: finish() then reads in stream order.)
+        self._done = None
+        if defer and not torch.cuda.is_current_stream_capturing():
             self._done = torch.cuda.Event()
             self._done.record()
 
     def finish(self):
+        import torch
         if self._done is not None:
             self._done.synchronize()
-            total, mx, mask, n_fb = self._host.tolist()
+            with torch.cuda.stream(_read_stream(self.info.device)):  # tolist() returns when the copy is done
+                total, mx, mask, n_fb = self.info.tolist()
         else:
             total, mx, mask, n_fb = self.info.tolist()
         out = self.out[:max(total, 4)].clone() if self.compact else self.out
         return DeviceEncodedColumn(out, self.meta, self.n, self.layout, total, mx, mask), self.schemes, n_fb
+
+
+_READ_STREAMS: dict = {}
+
+
+def _read_stream(device):
+    """The stream, one per device, on which finished encodes' info words are
+    read (blocking copies of 32 bytes; nothing is left behind on it)."""
+    import torch
+    s = _READ_STREAMS.get(device)
+    return s if s is not None else _READ_STREAMS.setdefault(device, torch.cuda.Stream(device))
 
 
 def encode_column_learned_gpu(values, params, threshold: float = 0.9, kappa: float = 0.0,
@@ -310,7 +320,7 @@ def encode_column_learned_gpu(values, params, threshold: float = 0.9, kappa: flo
                                        out.data_ptr(), bound + 4, meta.data_ptr(), info.data_ptr(), schemes.data_ptr(),
                                        ws.data_ptr(), ws_bytes, _lib.stream_handle()),
           "fls_encode_learned_gpu")
-    pending = PendingEncode(out, meta, info, schemes, n, layout, compact)
+    pending = PendingEncode(out, meta, info, schemes, n, layout, compact, defer)
     return pending if defer else pending.finish()
 
 
