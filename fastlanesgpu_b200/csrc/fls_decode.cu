@@ -213,27 +213,54 @@ fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_wor
 struct NoState {};
 
 // Decode to HBM.  Values of a vector are written as 32 coalesced 128-byte rows
-// with streaming stores; transposed columns can instead be reordered through a
-// padded shared-memory tile (33 words per chunk, conflict-free) into original
-// order.
+// with streaming stores; transposed columns can instead be reordered through
+// shared memory into original order.
+//
+// The reordering buffer holds chunk c (32 consecutive values) at words 32 c ..
+// 32 c + 31, its groups of four exchanged by c mod 8 and turned inside by c /
+// 8, so that a lane's column of chunk positions falls on 32 different banks
+// and four consecutive values still leave by one 16-byte read and one 16-byte
+// store: 48 memory instructions per vector instead of 96 with padded rows
+// (67 M DELTA values in original order: 59.4 -> 58.4 us, 50 M RLE 47.6 ->
+// 46.3).
 struct DecodeOp {
 	static constexpr uint32_t kWarps = 16;
 	uint32_t flight_share() const { return original ? 2u : 3u; }
 	using State = NoState;
 	uint32_t* out;
 	uint32_t  original;
+	uint32_t  wide; // out is 16-byte aligned
 	__device__ void process(State&, const ColumnVec& cv, uint32_t lane, const ColumnCfg&) const {
 		uint32_t vals[32];
 		dev::decode_vals(cv.s, cv.vi, cv.dict, lane, vals);
 		uint32_t* dst = out + cv.v * 1024u;
-		uint32_t* tb  = cv.extra;
 		if (original) {
-			const uint32_t cb = 33u * dev::chunk_of_lane(lane);
+			uint32_t*      tb = cv.extra;
+			const uint32_t c = dev::chunk_of_lane(lane), turn = c >> 3, swap = (c & 7u) << 2;
 #pragma unroll
-			for (uint32_t r = 0; r < 32; ++r) { tb[cb + dev::step_of_row(r)] = vals[r]; }
+			for (uint32_t r = 0; r < 32; ++r) {
+				const uint32_t t = dev::step_of_row(r);
+				tb[32u * c + ((t & 28u) ^ swap) + (((t & 3u) + turn) & 3u)] = vals[r];
+			}
 			__syncwarp();
+			if (wide) {
 #pragma unroll
-			for (uint32_t r = 0; r < 32; ++r) { dev::st_stream(dst + 32u * r + lane, tb[33u * r + lane]); }
+				for (uint32_t m = 0; m < 8; ++m) { // values 128 m + 4 lane .. + 3: chunk 4 m + lane / 8, group lane mod 8
+					const uint32_t k = 4u * m + (lane >> 3);
+					const uint4    q = *reinterpret_cast<const uint4*>(tb + 32u * k + (((lane & 7u) ^ (k & 7u)) << 2));
+					const uint32_t e[4] = {q.x, q.y, q.z, q.w};
+					// turned by k / 8 = m / 2
+					__stcs(reinterpret_cast<uint4*>(dst + 128u * m + 4u * lane),
+					       make_uint4(e[(m >> 1) & 3u], e[((m >> 1) + 1u) & 3u], e[((m >> 1) + 2u) & 3u],
+					                  e[((m >> 1) + 3u) & 3u]));
+				}
+			} else {
+#pragma unroll
+				for (uint32_t r = 0; r < 32; ++r) {
+					dev::st_stream(dst + 32u * r + lane,
+					               tb[32u * r + ((lane & 28u) ^ ((r & 7u) << 2)) + (((lane & 3u) + (r >> 3)) & 3u)]);
+				}
+			}
 			__syncwarp();
 		} else {
 #pragma unroll
@@ -488,7 +515,8 @@ fls_status fls_decode_u32(const fls_column* col, uint32_t* d_out, uint32_t order
 	DecodeOp op {};
 	op.out      = d_out;
 	op.original = orig ? 1u : 0u;
-	return launch_column(*col, op, orig ? kTBufWords : 0u, st);
+	op.wide     = (reinterpret_cast<uintptr_t>(d_out) & 15u) == 0 ? 1u : 0u;
+	return launch_column(*col, op, orig ? 1024u : 0u, st);
 }
 
 fls_status fls_decode_sum_u32(const fls_column* col, uint64_t* d_sum, fls_stream_t stream) {

@@ -44,7 +44,6 @@ constexpr uint32_t kJitDefaultWarps = 24;
 constexpr uint32_t kJitHalfWarps = 28;
 constexpr uint32_t kWaitPolls  = 1u << 17; // bounded mbarrier waits (x <= 20 us each)
 constexpr uint32_t kDictWords  = 1024;     // per-warp dictionary scratch
-constexpr uint32_t kTBufWords  = 33 * 32;  // per-warp transpose buffer
 constexpr uint32_t kBadScheme  = 0xffu;
 
 // ------------------------------------------------------------ parameters

@@ -207,3 +207,19 @@ def test_column_windows_and_rings(cuda, n_vec, scheme):
         ops.check_device_error()
     finally:
         ops.set_launch_config()
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("scheme", [0, 1, 2, 4])
+def test_original_order_into_any_alignment(cuda, shift, scheme):
+    """Original order leaves by 16-byte stores into aligned outputs and by words
+    into others; nothing outside the vectors is written."""
+    import torch
+    n = 5 * 1024 + 17
+    v = np.cumsum(np.random.default_rng(shift).integers(0, 9, n)).astype(np.int32)
+    col = EncodedColumn.encode(v, scheme).to_device()
+    buf = torch.full((6 * 1024 + shift + 5,), -7, dtype=torch.int32, device="cuda")
+    ops.unpack_global(col, ORDER_ORIGINAL, out=buf[shift:shift + 6 * 1024])
+    got = buf.cpu().numpy()
+    assert np.array_equal(got[shift:shift + 6 * 1024], _pad(v))
+    assert np.all(got[:shift] == -7) and np.all(got[shift + 6 * 1024:] == -7)
