@@ -10,9 +10,9 @@
 // each 128-byte row, which holds 32/T consecutive lanes, and extracts row r
 // of all of them at once (SIMD within a register: every lane of a word has
 // the same bit offset r*bw, so one shift and a per-lane mask serve all; the
-// base is added lane-wise without carries between lanes), at constant widths.  64-bit lanes: a
-// half-warp per vector, one lane per thread.  Both read and write 128-byte
-// rows per instruction.
+// base is added lane-wise without carries between lanes), at constant widths.
+// 64-bit lanes: a half-warp per vector, one lane per thread.  Both read and
+// write 128-byte rows per instruction.
 #include <cuda_runtime.h>
 
 #include <algorithm>
