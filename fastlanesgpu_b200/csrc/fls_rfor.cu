@@ -18,6 +18,9 @@
 //   4. a lane writes four consecutive positions at a time: the first is in run
 //      popc(mask bits up to it) - 1, each next one a run further where its bit
 //      is set; the values are gathered from shared memory.
+// Runs of length 0 cover no position: they add nothing to the sum and, to
+// memory, set no bit and keep no value (the values kept are those of the runs
+// that have a bit, in order).
 // A tile whose block is inconsistent is skipped and flagged, never read past
 // its stream.
 //
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(kRforWarps * 32, 6) rfor_kernel(const __grid_c
 		// runs do not cover it exactly is found out at the end: nothing of it
 		// has been added or written by then).
 		uint32_t           start = 0; // of the next 32 runs
+		[[maybe_unused]] uint32_t empty = 0; // runs of length 0 before them
 		unsigned long long part  = 0;
 		bool               fits  = true;
 		for (uint32_t i = 0; 32u * i < cnt; ++i) {
@@ -178,9 +182,17 @@ __global__ void __launch_bounds__(kRforWarps * 32, 6) rfor_kernel(const __grid_c
 			if constexpr (SUM) {
 				// the run's positions below `live`
 				part += static_cast<unsigned long long>(v) * (min(pos + l, live) - min(pos, live));
-			} else if (mine) {
-				vals[k] = v;
-				if (pos < kTile) { atomicOr(&words[pos >> 5].x, 1u << (pos & 31u)); } // a run of length 0 may end the tile
+			} else {
+				uint32_t       at   = k - empty;
+				const uint32_t none = __ballot_sync(0xffffffffu, mine && l == 0u);
+				if (none) { // not in this library's streams
+					at -= __popc(none & ((1u << lane) - 1u));
+					empty += __popc(none);
+				}
+				if (l != 0u && pos < kTile) { // past the tile: found out below
+					vals[at] = v;
+					atomicOr(&words[pos >> 5].x, 1u << (pos & 31u));
+				}
 			}
 			start += __shfl_sync(0xffffffffu, incl, 31);
 			if (!__all_sync(0xffffffffu, fits)) { break; }

@@ -240,7 +240,8 @@ fls_status fls_column_open_container(const void* buf, uint64_t bytes, fls_column
  * lengths) and of (n+511)/512 + 1 words (each offsets array).
  * fls_rfor_decode_u32 / fls_rfor_decode_sum_u32 (device): one warp per tile;
  * a tile whose block is inconsistent (counts, widths, offsets, run lengths
- * not summing to the tile) is skipped and flagged (fls_check_device_error). */
+ * not summing to the tile) is skipped and flagged (fls_check_device_error).
+ * A run of length 0, which this encoder never writes, covers no row. */
 typedef struct fls_rfor_column {
 	const uint32_t* values;      /* device: value stream        */
 	const uint32_t* run_lengths; /* device: run-length stream   */

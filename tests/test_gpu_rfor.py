@@ -143,3 +143,43 @@ def test_rfor_rows_and_alignment(cuda, n, mean_run):
         assert np.all(got[:shift] == -1) and np.all(got[shift + n:] == -1)
     assert int(ops.rfor_decode_sum(col).cpu()[0]) == int(vals.view(np.uint32).astype(np.uint64).sum())
     ops.check_device_error()
+
+
+def _block(x, bw):
+    """A block of a stream: minimum 0, bw in every byte, count, fields LSB first."""
+    bits = "".join(format(int(v), f"0{bw}b")[::-1] for v in x)
+    bits += "0" * (-len(bits) % 32)
+    return [0, bw * 0x01010101, len(x)] + [int(bits[i:i + 32][::-1], 2) for i in range(0, len(bits), 32)]
+
+
+EMPTY_RUNS = {
+    "first": [0, 512], "second": [2, 0, 510], "middle": [100, 0, 200, 0, 0, 212], "last": [300, 212, 0],
+    "most": [0] * 31 + [1] + [0] * 200 + [256, 0, 255] + [0] * 277, "group-edge": [8] * 31 + [0, 0] + [8] * 33,
+    "each-other": [2, 0] * 256, "trailing-group": [16] * 32 + [0] * 40,
+}
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_empty_runs_cover_no_row(cuda, shift):
+    """Runs of length 0, which no encoder here writes but the format holds:
+    before, between, after and instead of others, on both sides of a group of
+    32 runs; decode and sum expand the runs that are there."""
+    import torch
+    vs, rs, vo, ro, want = [512, 4, 0, 0], [512, 4, 0, 0], [], [], []
+    for i, (name, lens) in enumerate(EMPTY_RUNS.items()):
+        assert sum(lens) == 512 and len(lens) <= 512, name
+        vals = np.arange(1, len(lens) + 1) * 3 + 1000 * i
+        vo.append(len(vs))
+        ro.append(len(rs))
+        vs += _block(vals, 17)
+        rs += _block(lens, 10)
+        want.append(np.repeat(vals, lens))
+    want = np.concatenate(want).astype(np.int32)
+    u32 = lambda x: np.array(x, np.uint64).astype(np.uint32)  # noqa: E731
+    for n in (want.size, want.size - 300):
+        d = RforColumn(u32(vs), u32(rs), u32(vo + [len(vs)]), u32(ro + [len(rs)]), n).to_device()
+        buf = torch.full((n + shift,), -1, dtype=torch.int32, device="cuda")
+        ops.rfor_decode(d, out=buf[shift:])
+        assert np.array_equal(buf[shift:].cpu().numpy(), want[:n])
+        assert int(ops.rfor_decode_sum(d).cpu()[0]) == int(want[:n].astype(np.int64).sum())
+    ops.check_device_error()
