@@ -11,8 +11,10 @@
 //   1. lane l takes runs l, l + 32, ...: 32 fields of a packed block fill
 //      exactly bw words, so a lane's fields all start at the same bit and its
 //      shift and mask are constants; a warp scan of the lengths per 32 runs
-//      gives each run's first position;
-//   2. the sum needs no more: a run adds its value times its length;
+//      gives each run's first position (a tile of many runs: contiguous chunks
+//      and one scan, see many_runs);
+//   2. the sum needs no more: a run adds its value times its length, and a
+//      whole tile's not even the positions;
 //   3. to memory, each lane writes its runs' values to shared memory and sets
 //      the bit of each run's first position in a 512-bit mask (16 words);
 //   4. a lane writes four consecutive positions at a time: the first is in run
@@ -53,21 +55,28 @@ __device__ __forceinline__ uint32_t packed_words(uint32_t count, uint32_t bw) {
 // k*bw, LSB first): word row i of bw words holds fields 32 i .. 32 i + 31.
 // Never reads past the block's last packed word.
 struct LaneFields {
-	const uint32_t* p;
+	const uint32_t *block, *p;
 	uint32_t        bw, sh, mask, next;
-	__device__ __forceinline__ LaneFields(const uint32_t* block, uint32_t width, uint32_t lane) {
+	__device__ __forceinline__ LaneFields(const uint32_t* words, uint32_t width, uint32_t lane) {
 		const uint32_t bit = lane * width;
-		p    = block + (bit >> 5);
-		bw   = width;
-		sh   = bit & 31u;
-		mask = width >= 32 ? 0xffffffffu : ((1u << width) - 1u);
-		next = sh + width > 32u ? 1u : 0u; // without a second word the first is read twice and masked off
+		block = words;
+		p     = words + (bit >> 5);
+		bw    = width;
+		sh    = bit & 31u;
+		mask  = width >= 32 ? 0xffffffffu : ((1u << width) - 1u);
+		next  = sh + width > 32u ? 1u : 0u; // without a second word the first is read twice and masked off
 	}
 	// Row i's field; the caller has checked that it is one of the block's.
 	__device__ __forceinline__ uint32_t get(uint32_t i) const {
 		if (bw == 0) { return 0u; } // warp-uniform
 		const uint32_t* q = p + i * bw;
 		return __funnelshift_r(__ldg(q), __ldg(q + next), sh) & mask;
+	}
+	// Field k, whichever lane's it is (a block of width 0 still has one word).
+	__device__ __forceinline__ uint32_t any(uint32_t k) const {
+		const uint32_t  bit = k * bw, s = bit & 31u;
+		const uint32_t* q = block + (bit >> 5);
+		return __funnelshift_r(__ldg(q), s + bw > 32u ? __ldg(q + 1) : 0u, s) & mask;
 	}
 };
 
@@ -128,14 +137,71 @@ __device__ __forceinline__ TileHead load_head(const RforParams& P, uint64_t t) {
 	return h;
 }
 
-// WIDE: the output is 16-byte aligned.
+// Tiles of more than kFewRuns runs: each lane takes a contiguous chunk of the
+// runs, so that a tile takes one scan, its words are all asked for by the first
+// run of the chunks, and neighbouring starts are marked by one lane after the
+// other.  32 runs at a time take a chain of five shuffles and a round trip to
+// memory per 32 runs, and their starts, close together, meet in a word or two,
+// one atomic after the other (16.8 M values, whole call, 32 at a time -> this:
+// to memory, runs of mean 2 57 -> 37 and 4 37 -> 27 us; 1 stays at 104, bound by
+// the bank conflicts of chunks of 16; sums 64 -> 53, 47 -> 41 and 31 -> 27 with
+// the whole tiles' sums below).  `total`: the positions covered; SUM (of the
+// positions below `live`) into part.  False where a run has length 0 or passes
+// the tile: nothing that counts is done then.
+constexpr uint32_t kFewRuns = 64;
+template <bool SUM>
+__device__ __forceinline__ bool many_runs(const LaneFields& vf, const LaneFields& rf, uint32_t vmin, uint32_t rmin,
+                                          uint32_t cnt, uint32_t live, uint32_t* vals, uint16_t* lens, uint2* words,
+                                          uint32_t lane, uint32_t& total, unsigned long long& part) {
+	const uint32_t chunk = (cnt + 31u) >> 5, k0 = min(cnt, lane * chunk), k1 = min(cnt, k0 + chunk);
+	uint32_t       own = 0, most = 0; // most: the largest length minus one
+	for (uint32_t k = k0; k < k1; ++k) {
+		const uint32_t l = rmin + rf.any(k);
+		if constexpr (!SUM) {
+			vals[k] = vmin + vf.any(k);
+			lens[k] = static_cast<uint16_t>(l);
+		}
+		most = max(most, l - 1u);
+		own += l;
+	}
+	if (!__all_sync(0xffffffffu, most < kTile)) {
+		__syncwarp(); // the values are written once more
+		return false;
+	}
+	uint32_t incl = own;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+		if (lane >= static_cast<uint32_t>(o)) { incl += x; }
+	}
+	total = __shfl_sync(0xffffffffu, incl, 31);
+	if (total == kTile) { // every run starts inside the tile
+		uint32_t pos = incl - own;
+		for (uint32_t k = k0; k < k1; ++k) {
+			if constexpr (SUM) {
+				const uint32_t l = rmin + rf.any(k);
+				part += static_cast<unsigned long long>(vmin + vf.any(k)) * (min(pos + l, live) - min(pos, live));
+				pos += l;
+			} else { // each lane reads back its own lengths
+				atomicOr(&words[pos >> 5].x, 1u << (pos & 31u));
+				pos += lens[k];
+			}
+		}
+	}
+	return true;
+}
+
+// WIDE: the output is 16-byte aligned.  To memory five CTAs share an SM: at six
+// the 40 registers a thread spill (runs of mean 16 20.6 -> 23.8 us).
 template <bool SUM, bool WIDE>
-__global__ void __launch_bounds__(kRforWarps * 32, 6) rfor_kernel(const __grid_constant__ RforParams P) {
+__global__ void __launch_bounds__(kRforWarps * 32, SUM ? 6 : 5) rfor_kernel(const __grid_constant__ RforParams P) {
 	__shared__ uint32_t s_vals[SUM ? 1 : kRforWarps][kTile];
 	__shared__ uint2    s_words[SUM ? 1 : kRforWarps][kTile / 32];
+	__shared__ uint16_t s_lens[SUM ? 1 : kRforWarps][kTile];
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	uint32_t*      vals  = s_vals[SUM ? 0 : warp];
 	uint2*         words = s_words[SUM ? 0 : warp];
+	uint16_t*      lens  = s_lens[SUM ? 0 : warp];
 	unsigned long long acc = 0;
 	const uint64_t total = static_cast<uint64_t>(gridDim.x) * kRforWarps;
 	const uint64_t first = static_cast<uint64_t>(blockIdx.x) * kRforWarps + warp;
@@ -156,46 +222,67 @@ __global__ void __launch_bounds__(kRforWarps * 32, 6) rfor_kernel(const __grid_c
 			if (lane < kTile / 32) { words[lane] = make_uint2(0u, 0u); }
 			__syncwarp();
 		}
-		// Runs 32 i + lane, until the tile's runs are used up (a tile whose
-		// runs do not cover it exactly is found out at the end: nothing of it
-		// has been added or written by then).
 		uint32_t           start = 0; // of the next 32 runs
-		[[maybe_unused]] uint32_t empty = 0; // runs of length 0 before them
 		unsigned long long part  = 0;
-		bool               fits  = true;
-		for (uint32_t i = 0; 32u * i < cnt; ++i) {
-			const uint32_t k    = 32u * i + lane;
-			const bool     mine = k < cnt;
-			uint32_t       l = 0, v = 0;
-			if (mine) {
-				l = rmin + rf.get(i);
-				v = vmin + vf.get(i);
+		bool               fits  = true, grouped = true;
+		if (SUM && live == kTile) {
+			// A whole tile's sum needs no positions: no scan, every read
+			// independent of the one before.
+			grouped        = false;
+			uint32_t cover = 0;
+#pragma unroll 4
+			for (uint32_t i = 0; 32u * i < cnt; ++i) {
+				if (32u * i + lane < cnt) {
+					const uint32_t l = rmin + rf.get(i), v = vmin + vf.get(i);
+					fits             = fits && l <= kTile;
+					cover += l;
+					part += static_cast<unsigned long long>(v) * l;
+				}
 			}
-			fits          = fits && l <= kTile; // sums of 32 lengths below stay far from 32 bits
-			uint32_t incl = l;
+			start = __reduce_add_sync(0xffffffffu, cover);
+		}
+		if (cnt > kFewRuns && grouped) {
+			grouped = !many_runs<SUM>(vf, rf, vmin, rmin, cnt, live, vals, lens, words, lane, start, part);
+		}
+		if (grouped) {
+			// Runs 32 i + lane, until the tile's runs are used up (a tile whose
+			// runs do not cover it exactly is found out at the end: nothing of
+			// it has been added or written by then).
+			[[maybe_unused]] uint32_t empty = 0; // runs of length 0 so far
+			for (uint32_t i = 0; 32u * i < cnt; ++i) {
+				const uint32_t k    = 32u * i + lane;
+				const bool     mine = k < cnt;
+				uint32_t       l = 0, v = 0;
+				if (mine) {
+					l = rmin + rf.get(i);
+					v = vmin + vf.get(i);
+				}
+				fits          = fits && l <= kTile; // sums of 32 lengths below stay far from 32 bits
+				uint32_t incl = l;
 #pragma unroll
-			for (int o = 1; o < 32; o <<= 1) {
-				const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
-				if (lane >= static_cast<uint32_t>(o)) { incl += x; }
-			}
-			const uint32_t pos = start + incl - l;
-			if constexpr (SUM) {
-				// the run's positions below `live`
-				part += static_cast<unsigned long long>(v) * (min(pos + l, live) - min(pos, live));
-			} else {
-				uint32_t       at   = k - empty;
-				const uint32_t none = __ballot_sync(0xffffffffu, mine && l == 0u);
-				if (none) { // not in this library's streams
-					at -= __popc(none & ((1u << lane) - 1u));
-					empty += __popc(none);
+				for (int o = 1; o < 32; o <<= 1) {
+					const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+					if (lane >= static_cast<uint32_t>(o)) { incl += x; }
 				}
-				if (l != 0u && pos < kTile) { // past the tile: found out below
-					vals[at] = v;
-					atomicOr(&words[pos >> 5].x, 1u << (pos & 31u));
+				const uint32_t pos = start + incl - l;
+				if constexpr (SUM) {
+					// the run's positions below `live`
+					part += static_cast<unsigned long long>(v) * (min(pos + l, live) - min(pos, live));
+				} else {
+					uint32_t       at   = k - empty;
+					const uint32_t none = __ballot_sync(0xffffffffu, mine && l == 0u);
+					if (none) { // not in this library's streams
+						at -= __popc(none & ((1u << lane) - 1u));
+						empty += __popc(none);
+					}
+					if (l != 0u && pos < kTile) { // past the tile: found out below
+						vals[at] = v;
+						atomicOr(&words[pos >> 5].x, 1u << (pos & 31u));
+					}
 				}
+				start += __shfl_sync(0xffffffffu, incl, 31);
+				if (!__all_sync(0xffffffffu, fits)) { break; }
 			}
-			start += __shfl_sync(0xffffffffu, incl, 31);
-			if (!__all_sync(0xffffffffu, fits)) { break; }
 		}
 		if (start != kTile || !__all_sync(0xffffffffu, fits)) { // the runs must cover the tile exactly
 			if (lane == 0) { raise_err(P.err, kErrBadMeta); }
@@ -266,7 +353,7 @@ fls_status rfor_launch(const fls_rfor_column* col, uint32_t* d_out, uint64_t* d_
 		return s;
 	}
 	const uint32_t grid = static_cast<uint32_t>(
-	    std::min<uint64_t>((P.n_tiles + kRforWarps - 1) / kRforWarps, static_cast<uint64_t>(di.sms) * 6u)); // resident
+	    std::min<uint64_t>((P.n_tiles + kRforWarps - 1) / kRforWarps, static_cast<uint64_t>(di.sms) * (d_sum ? 6u : 5u))); // resident
 	if (d_sum) {
 		rfor_kernel<true, false><<<grid, kRforWarps * 32, 0, st>>>(P);
 	} else if ((reinterpret_cast<uintptr_t>(d_out) & 15u) == 0) {

@@ -183,3 +183,21 @@ def test_empty_runs_cover_no_row(cuda, shift):
         assert np.array_equal(buf[shift:].cpu().numpy(), want[:n])
         assert int(ops.rfor_decode_sum(d).cpu()[0]) == int(want[:n].astype(np.int64).sum())
     ops.check_device_error()
+
+
+def test_tiles_of_every_run_count(cuda):
+    """Tiles of 1..512 runs cut at random, so that both sides of every group of
+    32 runs and of the count that changes the kernel's path are met, with the
+    last tile whole and partial."""
+    g = np.random.default_rng(64)
+    tiles = []
+    for count in g.permutation(np.arange(1, 513)):
+        cuts = np.sort(g.permutation(511)[:count - 1]) + 1
+        lens = np.diff(np.concatenate([[0], cuts, [512]]))
+        tiles.append(np.repeat(g.integers(0, 1 << 20, count) * 2 + np.arange(count) % 2, lens))
+    vals = np.concatenate(tiles).astype(np.int32)
+    for n in (vals.size, vals.size - 1, vals.size - 300):
+        d = RforColumn.encode(vals[:n]).to_device()
+        assert np.array_equal(ops.rfor_decode(d).cpu().numpy(), vals[:n])
+        assert int(ops.rfor_decode_sum(d).cpu()[0]) == int(vals[:n].astype(np.int64).sum())
+    ops.check_device_error()
