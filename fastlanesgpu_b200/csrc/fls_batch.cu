@@ -122,14 +122,18 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 1) batch_kernel(const __grid_c
 	__syncwarp();
 	const uint64_t pol   = dev::l2_evict_first_policy();
 	uint32_t       phase = 0, st = 0; // running stage / phase across items
-	// the piece after the current one is taken while that one is worked on
-	unsigned long long next = 0;
-	if (lane == 0) { next = atomicAdd(P.counter, 1ull); }
+	// Every warp's first piece is its own number; the piece after the current
+	// one is taken from the counter while that one is worked on.  (With the
+	// first from the counter too, warps that start early take two pieces of a
+	// batch that has one for each: 8 columns of 2^14..2^18 values in items of
+	// one vector: 18 us before pieces, 22 so, now 19.)
+	const unsigned long long warps = static_cast<unsigned long long>(gridDim.x) * P.warps;
+	unsigned long long       next  = static_cast<unsigned long long>(blockIdx.x) * P.warps + warp;
 	for (;;) {
 		const uint64_t piece = __shfl_sync(0xffffffffu, next, 0);
 		if (piece >= P.n_pieces) { break; }
-		if (lane == 0) { next = atomicAdd(P.counter, 1ull); }
-		const uint64_t    item = piece / P.pieces_per_item;
+		if (lane == 0) { next = warps + atomicAdd(P.counter, 1ull); }
+		const uint64_t    item = piece >> 32 ? piece / P.pieces_per_item : static_cast<uint32_t>(piece) / P.pieces_per_item;
 		uint4             it   = P.items[item];
 		it.y += static_cast<uint32_t>(piece - item * P.pieces_per_item) * P.piece;
 		if (it.y >= it.z) { continue; } // a shorter item has fewer pieces

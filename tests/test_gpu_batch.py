@@ -171,3 +171,16 @@ def test_batch_sums_at_the_word_bound(cuda, bits, top):
     for i, q in enumerate(qs):
         assert tuple(got[i]) == _want([v] * 5, q)
     ops.check_device_error()
+
+
+@pytest.mark.parametrize("n_vec", [1, 147, 148, 149, 148 * 2 + 1, 148 * 16 - 1, 148 * 16, 148 * 16 + 1])
+def test_batch_fewer_and_more_pieces_than_warps(cuda, n_vec):
+    """One-vector pieces around one per SM and one per warp of a full grid:
+    every piece is done once, run after run."""
+    v = np.random.default_rng(n_vec).integers(-9, 1 << 11, n_vec * 1024 - 3).astype(np.int32)
+    qs = [(0, -9, 800, 0), (0, 3, 3, 0), (0, -2**31, 2**31 - 1, 0)]
+    b = Batch([EncodedColumn.encode(v, 0).to_device()], qs, chunk_vectors=1)
+    for _ in range(3):
+        got = b.run().cpu().numpy()
+        assert [tuple(r) for r in got] == [_want([v], q) for q in qs]
+    ops.check_device_error()
