@@ -180,21 +180,26 @@ def build_pht(keys, ht_len: int, vals=None, filt=None, filter_eq: int = 1, keys_
     """Selective perfect-hash table on device int32 columns: PHT_1 (vals None,
     ht_len slots) or PHT_2 (2*ht_len slots).  Rows with filt == filter_eq, or,
     with ranges=[(lo, hi)] (one or two inclusive ranges), rows whose filt lies
-    in one of them."""
+    in one of them.  out: a contiguous tensor of at least the table's bytes, all
+    of it zeroed and its first words filled."""
     import torch
     size = ht_len if vals is None else 2 * ht_len
+    name = "fls_pht_build_zeroed"  # zeroes a table's slots and builds
     if out is None:
         out = torch.empty(size, dtype=torch.int32, device=keys.device)
-    elif out.numel() != size or out.dtype != torch.int32 or not out.is_contiguous():
-        out.zero_()  # the library zeroes the ht_len slots of a table that is just as large
+    elif not out.is_contiguous() or out.numel() * out.element_size() < 4 * size:
+        raise ValueError(f"out must be contiguous and hold at least {size} int32 words")
+    elif out.numel() != size or out.dtype != torch.int32:
+        out.zero_()  # all of it, not only the table's slots
+        name = "fls_pht_build_ranges"
     if ranges is None:
         ranges = [(filter_eq, filter_eq)]
     if not 1 <= len(ranges) <= 2:
         raise ValueError("one or two filter ranges")
     (lo0, hi0), (lo1, hi1) = ranges[0], ranges[1] if len(ranges) == 2 else (1, 0)
-    check(lib().fls_pht_build_zeroed(0 if filt is None else filt.data_ptr(), lo0, hi0, lo1, hi1, keys.data_ptr(),
-                                     0 if vals is None else vals.data_ptr(), keys.numel(), out.data_ptr(), ht_len,
-                                     keys_min, _stream()), "fls_pht_build_zeroed")
+    check(getattr(lib(), name)(0 if filt is None else filt.data_ptr(), lo0, hi0, lo1, hi1, keys.data_ptr(),
+                               0 if vals is None else vals.data_ptr(), keys.numel(), out.data_ptr(), ht_len,
+                               keys_min, _stream()), name)
     return out
 
 
