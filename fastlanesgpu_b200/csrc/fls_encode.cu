@@ -37,6 +37,7 @@ constexpr uint32_t kNetWords     = sel::kPadded + sel::kBuckets / 4u; // offset 
 static_assert(kEncWarpWords % 4 == 0 && kEncWarpWords >= kNetWords + sel::WarpNet::kScratch, "the warp's words");
 constexpr uint32_t kKeyedBits    = 22;               // widest range whose sort keys carry the value's index
 constexpr uint32_t kPollLimit   = 1u << 22;          // bounded waits on other tiles (each poll is an L2 round trip)
+constexpr uint32_t kAloneRounds = 64;                // idle rounds after which the scan looks whether any tile is taken
 
 struct EncParams {
 	const int32_t* values;
@@ -53,6 +54,7 @@ struct EncParams {
 	uint32_t*      counter; // next ticket, CTAs done (zeroed before the launch)
 	uint64_t*      reports; // per tile (zeroed before the launch)
 	uint64_t*      offsets; // per tile (zeroed before the launch)
+	uint32_t       scan_polls, tile_polls; // limits of the scan's and of a tile's wait
 	uint64_t*      info;    // [0] total words, [1] max vector words, [2] scheme mask; learned: [3] fallbacks
 	uint32_t*      err;
 	// learned selection
@@ -82,26 +84,39 @@ __device__ __forceinline__ void tile_store(uint64_t* p, uint64_t v) {
 	asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// The scan of the tiles' reports.
+struct ScanState {
+	uint64_t pos, run; // tiles answered, their words
+	uint32_t mx, mask;
+};
+
 // One warp: takes the tiles' reports in order, answers each with its offset
 // and leaves the column's totals in info.  A round reads kScanGroups x 32
-// reports, all loads in flight, and answers those that are there.  Tiles are
-// taken in order by running CTAs, so the next report always comes; should
-// kPollLimit rounds bring none, the tiles still waiting are told so.
+// reports, all loads in flight, and answers those that are there.  Returns 0
+// when nothing is left to do.
+//
+// Only tiles that running CTAs have taken are waited for, so the next report
+// always comes; should scan_polls rounds bring none all the same, the tiles
+// still waiting are told so.  A tile that no CTA has taken may be long in
+// coming: other work may hold every other place on the GPU for as long as it
+// likes.  So where all tiles taken are answered, the scan takes the next one
+// (by compare and swap: it is the next to be answered too) and returns its
+// ticket, with its own state in S, for the CTA to encode it: one resident CTA
+// finishes the column.
 //
 // Why one warp: a look-back by every tile over those before it (256 reports
 // per round trip) cost the tiles 4-7 us each on a column of 733 tiles, since
 // all of a GPU's tiles finish planning together and walk the same states.
 constexpr uint32_t kScanGroups = 8;
-__device__ void scan_tiles(const uint64_t* reports, uint64_t* offsets, uint64_t n_tiles, uint64_t* info, uint32_t* err,
-                           uint32_t lane) {
-	uint64_t pos = 0, run = 0;
-	uint32_t mx = 0, mask = 0, idle = 0;
-	while (pos < n_tiles) {
+__device__ __forceinline__ uint32_t scan_tiles(const EncParams& P, ScanState& S, uint32_t alone_rounds, uint32_t lane) {
+	uint64_t pos = S.pos, run = S.run;
+	uint32_t mx = S.mx, mask = S.mask, idle = 0;
+	while (pos < P.n_tiles) {
 		uint64_t s[kScanGroups];
 #pragma unroll
 		for (uint32_t g = 0; g < kScanGroups; ++g) {
 			const uint64_t t = pos + 32u * g + lane;
-			s[g]             = t < n_tiles ? tile_load(reports + t) : 0ull;
+			s[g]             = t < P.n_tiles ? tile_load(P.reports + t) : 0ull;
 		}
 		const uint64_t pos0 = pos;
 		bool           more = true;
@@ -119,7 +134,7 @@ __device__ void scan_tiles(const uint64_t* reports, uint64_t* offsets, uint64_t 
 				const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
 				if (lane >= static_cast<uint32_t>(o)) { incl += y; }
 			}
-			if (mine) { tile_store(offsets + pos + lane, kTileMark | (run + incl - w)); }
+			if (mine) { tile_store(P.offsets + pos + lane, kTileMark | (run + incl - w)); }
 			run += __shfl_sync(0xffffffffu, incl, 31);
 			mx = max(mx, hi & 0xffffu);
 			mask |= hi >> 16;
@@ -127,22 +142,32 @@ __device__ void scan_tiles(const uint64_t* reports, uint64_t* offsets, uint64_t 
 			more = n == 32u;
 		}
 		idle = pos == pos0 ? idle + 1u : 0u;
-		if (idle == kPollLimit) {
-			if (lane == 0) {
-				atomicOr(err, kErrTimeout);
-				info[0] = info[1] = info[2] = 0;
+		if (idle >= alone_rounds && idle % kAloneRounds == alone_rounds % kAloneRounds) {
+			const uint32_t next = static_cast<uint32_t>(pos) + 1u; // the ticket after those of the tiles answered
+			uint32_t       had  = 0;
+			if (lane == 0) { had = atomicCAS(P.counter, next, next + 1u); }
+			if (__shfl_sync(0xffffffffu, had, 0) == next) {
+				S = ScanState {pos, run, __reduce_max_sync(0xffffffffu, mx), __reduce_or_sync(0xffffffffu, mask)};
+				return next;
 			}
-			for (uint64_t t = pos + lane; t < n_tiles; t += 32u) { tile_store(offsets + t, kTileLost); }
-			return;
+		}
+		if (idle >= P.scan_polls) {
+			if (lane == 0) {
+				atomicOr(P.err, kErrTimeout);
+				P.info[0] = P.info[1] = P.info[2] = 0;
+			}
+			for (uint64_t t = pos + lane; t < P.n_tiles; t += 32u) { tile_store(P.offsets + t, kTileLost); }
+			return 0;
 		}
 	}
 	mx   = __reduce_max_sync(0xffffffffu, mx);
 	mask = __reduce_or_sync(0xffffffffu, mask);
 	if (lane == 0) {
-		info[0] = run;
-		info[1] = mx;
-		info[2] = mask;
+		P.info[0] = run;
+		P.info[1] = mx;
+		P.info[2] = mask;
 	}
+	return 0;
 }
 
 __device__ __forceinline__ uint32_t bits_of(uint32_t v) { return v ? 32u - __clz(v) : 0u; }
@@ -551,6 +576,129 @@ __device__ __forceinline__ void write_vector(const EncParams& P, uint64_t v, con
 	pack_lane(x, bw, out + skip, lane);
 }
 
+// What the warps of a CTA share on a tile.
+struct TileShared {
+	uint32_t words[kEncWarps], mask[kEncWarps];
+	uint64_t offset;
+};
+
+// The scanning CTA's own tile is the next to be answered.
+__device__ __forceinline__ void offset_alone(TileShared& T, ScanState* scan, uint64_t own, uint32_t lane) {
+	const uint32_t hi = static_cast<uint32_t>(own >> 32) & 0x7fffffffu;
+	if (lane == 0) { T.offset = kTileMark | scan->run; }
+	__syncwarp();
+	scan->pos += 1u;
+	scan->run += static_cast<uint32_t>(own);
+	scan->mx = max(scan->mx, hi & 0xffffu);
+	scan->mask |= hi >> 16;
+}
+
+// One tile by the CTA; returns whether the warp's vector fell back to the
+// exhaustive choice.  ALONE: by the scanning CTA (scan: warp 0's state).
+template <bool LEARNED, bool ALONE>
+__device__ __forceinline__ bool encode_tile(const EncParams& P, uint64_t tile, int32_t* sv, const float* net,
+                                            TileShared& T, ScanState* scan, uint32_t warp, uint32_t lane) {
+	const uint64_t v    = tile * kEncWarps + warp;
+	const bool     live = v < P.n_vec;
+	Plan           p {};
+	uint32_t       words = 0;
+	int32_t        mn = 0, mx = 0;
+	sel::Counts    counts {};
+	uint32_t       scheme = 0;
+	bool           unsure = false;
+	if (live) { sel::stage_vector(P.values, P.n, v, sv, lane, mn, mx); }
+	// the vector this warp is likely to take next: from memory to L2
+	const uint64_t ahead = v + static_cast<uint64_t>(gridDim.x) * kEncWarps;
+	if ((ahead + 1u) * 1024u <= P.n) {
+		asm volatile("prefetch.global.L2 [%0];" ::"l"(P.values + ahead * 1024u + 32u * lane));
+	}
+	if constexpr (LEARNED) {
+		if (live) {
+			const float f = sel::vector_features(sv, mn, mx, reinterpret_cast<uint8_t*>(sv + sel::kPadded), lane, counts);
+			float       z[sel::kOut], top;
+			sel::WarpNet::forward(net, reinterpret_cast<float*>(sv + kNetWords), f, lane, z);
+			sel::softmax5(z);
+			scheme = static_cast<uint32_t>(sel::top_of(z, top));
+			unsure = top < P.threshold;
+			__syncwarp(); // the activations are read before the warp's words serve something else
+		}
+	} else if (live) {
+		scheme = P.schemes ? P.schemes[v] : P.scheme;
+		if (scheme >= FLS_N_SCHEMES) {
+			if (lane == 0) { atomicOr(P.err, kErrBadMeta); }
+			scheme = FLS_SCHEME_FOR;
+		}
+	}
+	if (live) {
+		p     = plan_vector<LEARNED>(P, v, sv, lane, mn, mx, scheme, counts, unsure);
+		words = payload_words(p.scheme, p.bw, p.aux);
+		if (LEARNED && P.picks && lane == 0) { P.picks[v] = static_cast<uint8_t>(scheme); }
+	}
+	if (lane == 0) {
+		T.words[warp] = words;
+		T.mask[warp]  = live ? 1u << p.scheme : 0u;
+	}
+	__syncthreads();
+	if (warp == 0) {
+		const uint32_t w = lane < kEncWarps ? T.words[lane] : 0u, m = lane < kEncWarps ? T.mask[lane] : 0u;
+		const uint64_t own = tile_report(__reduce_add_sync(0xffffffffu, w), __reduce_max_sync(0xffffffffu, w),
+		                                 __reduce_or_sync(0xffffffffu, m));
+		if (ALONE) {
+			offset_alone(T, scan, own, lane);
+		} else if (lane == 0) {
+			tile_store(P.reports + tile, own);
+			uint64_t got = 0;
+			for (uint32_t poll = 0; poll < P.tile_polls && got == 0ull; ++poll) { got = tile_load(P.offsets + tile); }
+			if (got == 0ull) {
+				atomicOr(P.err, kErrTimeout);
+				got = kTileLost;
+			}
+			T.offset = got;
+		}
+	}
+	__syncthreads();
+	const uint64_t before = T.offset;
+	if (live && before != kTileLost) {
+		uint64_t offset = before & ~kTileMark;
+		for (uint32_t w = 0; w < warp; ++w) { offset += T.words[w]; }
+		if (lane == 0) {
+			fls_vec_meta m;
+			m.offset  = offset;
+			m.base    = p.base;
+			m.scheme  = static_cast<uint8_t>(p.scheme);
+			m.bw      = static_cast<uint8_t>(p.bw);
+			m.aux     = static_cast<uint16_t>(p.aux);
+			P.meta[v] = m;
+		}
+		write_vector(P, v, p, sv, P.out + offset, lane);
+	}
+	__syncthreads(); // T is read before the next tile's
+	return unsure;
+}
+
+// The rest of the column by the scanning CTA, from the tile of `ticket` on, with
+// whatever tiles other CTAs have taken in between.  Returns the warp's
+// fallbacks.  Apart from the kernel's loop, so that the registers of the scan and
+// of a tile stay apart there (33.5 M values as a dictionary, kernel: 264 us
+// without it, 270 with it, 276 where the scan went back into the loop).
+template <bool LEARNED>
+__device__ __forceinline__ uint32_t encode_alone(const EncParams& P, uint32_t ticket, int32_t* sv, const float* net,
+                                              TileShared& T, uint32_t& s_tile, ScanState scan, uint32_t warp,
+                                              uint32_t lane) {
+	uint32_t fallbacks = 0;
+	while (ticket != 0u) {
+		fallbacks += encode_tile<LEARNED, true>(P, ticket - 1u, sv, net, T, &scan, warp, lane) ? 1u : 0u;
+		if (warp == 0) {
+			ticket = scan_tiles(P, scan, 1u, lane); // still alone: the next tile at once
+			if (lane == 0) { s_tile = ticket; }
+		}
+		__syncthreads();
+		ticket = s_tile;
+		__syncthreads();
+	}
+	return fallbacks;
+}
+
 // Bounded by the per-vector work of planning (DICT: the sort; LEARNED: the
 // statistics and the network, about 6 us of a round of 24 vectors per SM) and,
 // in columns of few rounds, by the round trip of a tile's offset, 2-4 us.
@@ -568,9 +716,9 @@ __device__ __forceinline__ void write_vector(const EncParams& P, uint64_t v, con
 template <bool LEARNED>
 __global__ void __launch_bounds__(kEncWarps * 32, 3) enc_kernel(const __grid_constant__ EncParams P) {
 	extern __shared__ __align__(16) int32_t esmem[];
-	__shared__ uint32_t s_tile;
-	__shared__ uint32_t s_words[kEncWarps], s_mask[kEncWarps];
-	__shared__ uint64_t s_offset;
+	__shared__ uint32_t   s_tile;
+	__shared__ TileShared s_shared;
+	__shared__ ScanState  s_scan; // of the CTA with the first ticket
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	int32_t*       sv   = esmem + warp * kEncWarpWords;
 	float*         net  = reinterpret_cast<float*>(esmem + kEncWarps * kEncWarpWords); // LEARNED
@@ -582,85 +730,23 @@ __global__ void __launch_bounds__(kEncWarps * 32, 3) enc_kernel(const __grid_con
 		if (threadIdx.x == 0) { s_tile = atomicAdd(P.counter, 1u); }
 		__syncthreads();
 		if (s_tile == 0u) { // the first ticket: this CTA adds up the tiles
-			if (warp == 0) { scan_tiles(P.reports, P.offsets, P.n_tiles, P.info, P.err, lane); }
+			__syncthreads(); // s_tile is read
+			if (warp == 0) {
+				if (lane == 0) { s_scan = ScanState {}; }
+				__syncwarp();
+				const uint32_t ticket = scan_tiles(P, s_scan, kAloneRounds, lane);
+				if (lane == 0) { s_tile = ticket; }
+			}
+			__syncthreads();
 			break;
 		}
 		const uint64_t tile = s_tile - 1u;
 		if (tile >= P.n_tiles) { break; }
-		const uint64_t v    = tile * kEncWarps + warp;
-		const bool     live = v < P.n_vec;
-		Plan           p {};
-		uint32_t       words = 0;
-		int32_t        mn = 0, mx = 0;
-		sel::Counts    counts {};
-		uint32_t       scheme = 0;
-		bool           unsure = false;
-		if (live) { sel::stage_vector(P.values, P.n, v, sv, lane, mn, mx); }
-		// the vector this warp is likely to take next: from memory to L2
-		const uint64_t ahead = v + static_cast<uint64_t>(gridDim.x) * kEncWarps;
-		if ((ahead + 1u) * 1024u <= P.n) {
-			asm volatile("prefetch.global.L2 [%0];" ::"l"(P.values + ahead * 1024u + 32u * lane));
-		}
-		if constexpr (LEARNED) {
-			if (live) {
-				const float f = sel::vector_features(sv, mn, mx, reinterpret_cast<uint8_t*>(sv + sel::kPadded), lane, counts);
-				float       z[sel::kOut], top;
-				sel::WarpNet::forward(net, reinterpret_cast<float*>(sv + kNetWords), f, lane, z);
-				sel::softmax5(z);
-				scheme = static_cast<uint32_t>(sel::top_of(z, top));
-				unsure = top < P.threshold;
-				__syncwarp(); // the activations are read before the warp's words serve something else
-			}
-		} else if (live) {
-			scheme = P.schemes ? P.schemes[v] : P.scheme;
-			if (scheme >= FLS_N_SCHEMES) {
-				if (lane == 0) { atomicOr(P.err, kErrBadMeta); }
-				scheme = FLS_SCHEME_FOR;
-			}
-		}
-		if (live) {
-			p     = plan_vector<LEARNED>(P, v, sv, lane, mn, mx, scheme, counts, unsure);
-			words = payload_words(p.scheme, p.bw, p.aux);
-			if (LEARNED && P.picks && lane == 0) { P.picks[v] = static_cast<uint8_t>(scheme); }
-		}
-		fallbacks += unsure ? 1u : 0u;
-		if (lane == 0) {
-			s_words[warp] = words;
-			s_mask[warp]  = live ? 1u << p.scheme : 0u;
-		}
-		__syncthreads();
-		if (warp == 0) {
-			const uint32_t w = lane < kEncWarps ? s_words[lane] : 0u, m = lane < kEncWarps ? s_mask[lane] : 0u;
-			const uint64_t own = tile_report(__reduce_add_sync(0xffffffffu, w), __reduce_max_sync(0xffffffffu, w),
-			                                 __reduce_or_sync(0xffffffffu, m));
-			if (lane == 0) {
-				tile_store(P.reports + tile, own);
-				uint64_t got = 0;
-				for (uint32_t poll = 0; poll < kPollLimit && got == 0ull; ++poll) { got = tile_load(P.offsets + tile); }
-				if (got == 0ull) {
-					atomicOr(P.err, kErrTimeout);
-					got = kTileLost;
-				}
-				s_offset = got;
-			}
-		}
-		__syncthreads();
-		const uint64_t before = s_offset;
-		if (live && before != kTileLost) {
-			uint64_t offset = before & ~kTileMark;
-			for (uint32_t w = 0; w < warp; ++w) { offset += s_words[w]; }
-			if (lane == 0) {
-				fls_vec_meta m;
-				m.offset  = offset;
-				m.base    = p.base;
-				m.scheme  = static_cast<uint8_t>(p.scheme);
-				m.bw      = static_cast<uint8_t>(p.bw);
-				m.aux     = static_cast<uint16_t>(p.aux);
-				P.meta[v] = m;
-			}
-			write_vector(P, v, p, sv, P.out + offset, lane);
-		}
-		__syncthreads(); // s_words is read before the next tile's
+		fallbacks += encode_tile<LEARNED, false>(P, tile, sv, net, s_shared, nullptr, warp, lane) ? 1u : 0u;
+	}
+	// s_tile: past the last tile, or, in the scanning CTA, 0 or a tile to go on with
+	if (s_tile != 0u && s_tile <= P.n_tiles) {
+		fallbacks += encode_alone<LEARNED>(P, s_tile, sv, net, s_shared, s_tile, s_scan, warp, lane);
 	}
 	if constexpr (LEARNED) {
 		// The last CTA to get here reports the fallbacks of all.
@@ -680,10 +766,11 @@ uint64_t workspace_bytes_of(uint64_t n) {
 }
 
 // Checks the arguments both encoders share, fills in the rest of P and
-// launches the kernel: one memset of the tiles' states, one launch.
+// launches the kernel: one memset of the tiles' states, one launch.  max_ctas:
+// of the launch (0: as many as are resident).
 template <bool LEARNED>
 fls_status encode_launch(EncParams& P, uint64_t out_capacity_words, void* d_workspace, uint64_t workspace_bytes,
-                         cudaStream_t st, const std::string& who) {
+                         cudaStream_t st, const std::string& who, uint32_t max_ctas = 0) {
 	if (!P.values || !P.out || !P.meta || !P.info || !d_workspace || P.n == 0) {
 		return set_error(FLS_ERR_INVALID_ARG, who + ": null pointer or n == 0");
 	}
@@ -727,8 +814,8 @@ fls_status encode_launch(EncParams& P, uint64_t out_capacity_words, void* d_work
 		}
 	}
 	if ((s = cuda_check(cudaMemsetAsync(ws, 0, 16u + 16u * P.n_tiles, st), "cudaMemsetAsync")) != FLS_OK) { return s; }
-	const uint32_t grid =
-	    static_cast<uint32_t>(std::min<uint64_t>(P.n_tiles + 1u, static_cast<uint64_t>(di.sms) * 3u));
+	const uint32_t grid = static_cast<uint32_t>(
+	    std::min<uint64_t>(P.n_tiles + 1u, max_ctas ? max_ctas : static_cast<uint64_t>(di.sms) * 3u));
 	enc_kernel<LEARNED><<<grid, kEncWarps * 32, smem, st>>>(P);
 	count_launch();
 	return cuda_check(cudaGetLastError(), "enc_kernel launch");
@@ -758,6 +845,7 @@ fls_status fls_encode_column_gpu(const int32_t* d_values, uint64_t n, const uint
 	P.out     = d_out;
 	P.meta    = d_meta;
 	P.info    = d_info;
+	P.scan_polls = P.tile_polls = kPollLimit;
 	return encode_launch<false>(P, out_capacity_words, d_workspace, workspace_bytes,
 	                            reinterpret_cast<cudaStream_t>(stream), "fls_encode_column_gpu");
 }
@@ -784,8 +872,33 @@ fls_status fls_encode_learned_gpu(const int32_t* d_values, uint64_t n, const flo
 	P.threshold = threshold;
 	P.kappa     = kappa;
 	P.picks     = d_schemes;
+	P.scan_polls = P.tile_polls = kPollLimit;
 	return encode_launch<true>(P, out_capacity_words, d_workspace, workspace_bytes,
 	                           reinterpret_cast<cudaStream_t>(stream), "fls_encode_learned_gpu");
+}
+
+fls_status fls_selftest_encode_waits(const int32_t* d_values, uint64_t n, uint32_t scheme, const float* d_params,
+                                     uint32_t* d_out, uint64_t out_capacity_words, fls_vec_meta* d_meta,
+                                     uint64_t* d_info, void* d_workspace, uint64_t workspace_bytes, uint32_t ctas,
+                                     uint32_t scan_polls, uint32_t tile_polls, fls_stream_t stream) {
+	if (scheme >= FLS_N_SCHEMES || ctas == 0 || scan_polls > kPollLimit || tile_polls > kPollLimit) {
+		return set_error(FLS_ERR_INVALID_ARG, "fls_selftest_encode_waits: bad scheme, CTAs or limits");
+	}
+	EncParams P {};
+	P.values     = d_values;
+	P.n          = n;
+	P.scheme     = scheme;
+	P.layout     = FLS_LAYOUT_TRANSPOSED;
+	P.out        = d_out;
+	P.meta       = d_meta;
+	P.info       = d_info;
+	P.scan_polls = scan_polls;
+	P.tile_polls = tile_polls;
+	P.params     = d_params;
+	P.threshold  = 0.9f;
+	const auto st = reinterpret_cast<cudaStream_t>(stream);
+	return d_params ? encode_launch<true>(P, out_capacity_words, d_workspace, workspace_bytes, st, __func__, ctas)
+	                : encode_launch<false>(P, out_capacity_words, d_workspace, workspace_bytes, st, __func__, ctas);
 }
 
 } // extern "C"

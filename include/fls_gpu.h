@@ -125,6 +125,16 @@ fls_status fls_bind_error_word(fls_stream_t stream, uint32_t* d_words);
  * and raises the timeout bit, so the next fls_check_device_error returns
  * FLS_ERR_TIMEOUT; the context stays usable.  Nothing faults or hangs. */
 fls_status fls_selftest_bounded_wait(uint32_t polls, fls_stream_t stream);
+/* Self-test of the GPU encoder's waits (no reference counterpart):
+ * fls_encode_column_gpu with `scheme`, or, with d_params, fls_encode_learned_gpu
+ * at a threshold of 0.9 and kappa 0, both transposed, by at most `ctas` CTAs (1:
+ * as when other work holds the rest of the GPU) and with the encoder's two waits
+ * ended after scan_polls and tile_polls tries.  At 0 tries the encode is lost:
+ * the timeout bit is raised, and the context stays usable. */
+fls_status fls_selftest_encode_waits(const int32_t* d_values, uint64_t n, uint32_t scheme, const float* d_params,
+                                     uint32_t* d_out, uint64_t out_capacity_words, struct fls_vec_meta* d_meta,
+                                     uint64_t* d_info, void* d_workspace, uint64_t workspace_bytes, uint32_t ctas,
+                                     uint32_t scan_polls, uint32_t tile_polls, fls_stream_t stream);
 
 /* ------------------------------------------------- host encoders (CPU) */
 

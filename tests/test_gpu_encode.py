@@ -124,3 +124,43 @@ def test_gpu_encoder_offsets_over_many_tiles(cuda, n_vec):
     vals = (g.integers(0, 1 << 31, (n_vec, 1024)) >> g.integers(0, 31, (n_vec, 1))).astype(np.int32).reshape(-1)[:-11]
     schemes = np.where(g.integers(0, 50, n_vec) == 0, g.integers(0, 5, n_vec), 0).astype(np.uint8)
     _compare(vals, schemes, LAYOUT_TRANSPOSED)
+
+
+def _encode_waits(values, scheme=0, params=None, ctas=1, scan_polls=1 << 22, tile_polls=1 << 22):
+    """The encoder with few CTAs and short waits: (words, metadata, info)."""
+    import torch
+    from fastlanesgpu_b200._lib import check, lib
+    n = values.numel()
+    cap = int(lib().fls_encode_bound_words(n)) + 4
+    out = torch.full((cap,), -1, dtype=torch.int32, device="cuda")
+    meta = torch.full(((n + 1023) // 1024 * 4,), -1, dtype=torch.int32, device="cuda")
+    info = torch.full((4,), 99, dtype=torch.int64, device="cuda")
+    ws = torch.empty(int(lib().fls_encode_learned_workspace_bytes(n)), dtype=torch.uint8, device="cuda")
+    check(lib().fls_selftest_encode_waits(values.data_ptr(), n, scheme, params.data_ptr() if params is not None else None,
+                                          out.data_ptr(), cap, meta.data_ptr(), info.data_ptr(), ws.data_ptr(),
+                                          ws.numel(), ctas, scan_polls, tile_polls,
+                                          torch.cuda.current_stream().cuda_stream), "fls_selftest_encode_waits")
+    return out, meta, info.tolist()
+
+
+@pytest.mark.parametrize("ctas", [1, 2, 3])
+@pytest.mark.parametrize("n_vec", [1, 8, 9, 8 * 33 + 5, 8 * 300])
+def test_encoder_by_few_ctas(cuda, ctas, n_vec):
+    """However few CTAs of the encoder are on the GPU, one included, the column
+    is encoded whole and as by many, without a timeout."""
+    import torch
+    from fastlanesgpu_b200 import _lib
+    from fastlanesgpu_b200.column import encode_column_learned_gpu
+    n = n_vec * 1024 - 7
+    for scheme, name in enumerate(("uniform", "sorted", "runs", "constant", "zipf")):
+        v = torch.from_numpy(_families(n, n_vec)[name]).cuda()
+        want = encode_column_gpu(v, scheme)
+        out, meta, info = _encode_waits(v, scheme, ctas=ctas)
+        assert info[:3] == [want.payload_words, want.desc.max_vec_words, want.desc.scheme_mask]
+        assert torch.equal(out[:info[0]], want.data[:info[0]]) and torch.equal(meta, want.meta)
+    params = torch.randn(_lib.MLP_N_PARAMS, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n_vec))
+    want, _, fallbacks = encode_column_learned_gpu(v, params, threshold=0.9, kappa=0.0)
+    out, meta, info = _encode_waits(v, params=params, ctas=ctas)
+    assert info == [want.payload_words, want.desc.max_vec_words, want.desc.scheme_mask, fallbacks]
+    assert torch.equal(out[:info[0]], want.data[:info[0]]) and torch.equal(meta, want.meta)
+    ops.check_device_error()
