@@ -12,7 +12,7 @@ import os
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libfls_gpu.so")
 
-FLS_OK = 0
+FLS_OK, ERR_TIMEOUT = 0, 6
 STATUS_NAMES = {0: "FLS_OK", 1: "FLS_ERR_INVALID_ARG", 2: "FLS_ERR_BAD_BW", 3: "FLS_ERR_ALIGNMENT",
                 4: "FLS_ERR_CUDA", 5: "FLS_ERR_DEVICE", 6: "FLS_ERR_TIMEOUT", 7: "FLS_ERR_UNSUPPORTED",
                 8: "FLS_ERR_CAPACITY", 9: "FLS_ERR_NO_DEVICE"}

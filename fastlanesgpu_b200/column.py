@@ -251,10 +251,20 @@ def encode_column_gpu(values, schemes=0, layout: int = LAYOUT_TRANSPOSED, round4
                                       0 if per_vec else int(schemes), layout, int(round4), out.data_ptr(), bound + 4,
                                       meta.data_ptr(), info.data_ptr(), ws.data_ptr(), ws_bytes,
                                       _lib.stream_handle()), "fls_encode_column_gpu")
-    total, mx, mask = info.tolist()
+    total, mx, mask = _totals(info, "fls_encode_column_gpu")
     if compact:
         out = out[:max(total, 4)].clone()
     return DeviceEncodedColumn(out, meta, n, layout, total, mx, mask)
+
+
+def _totals(info, where: str) -> list:
+    """The encoder's info words, on the host.  A scheme mask of 0 is an encode
+    that was lost (a wait on the device ran out): an error, since its words and
+    metadata are not there."""
+    words = info.tolist()
+    if words[2] == 0:
+        raise _lib.FlsError(_lib.ERR_TIMEOUT, where, "the encode was lost (a wait on the device ran out)")
+    return words
 
 
 class PendingEncode:
@@ -279,9 +289,9 @@ class PendingEncode:
         if self._done is not None:
             self._done.synchronize()
             with torch.cuda.stream(_read_stream(self.info.device)):  # tolist() returns when the copy is done
-                total, mx, mask, n_fb = self.info.tolist()
+                total, mx, mask, n_fb = _totals(self.info, "fls_encode_learned_gpu")
         else:
-            total, mx, mask, n_fb = self.info.tolist()
+            total, mx, mask, n_fb = _totals(self.info, "fls_encode_learned_gpu")
         out = self.out[:max(total, 4)].clone() if self.compact else self.out
         return DeviceEncodedColumn(out, self.meta, self.n, self.layout, total, mx, mask), self.schemes, n_fb
 

@@ -52,6 +52,7 @@ struct EncParams {
 	fls_vec_meta*  meta;
 	uint64_t       n_tiles;
 	uint32_t*      counter; // next ticket, CTAs done (zeroed before the launch)
+	uint32_t*      lost;    // set by a tile that gave up waiting (zeroed before the launch)
 	uint64_t*      reports; // per tile (zeroed before the launch)
 	uint64_t*      offsets; // per tile (zeroed before the launch)
 	uint32_t       scan_polls, tile_polls; // limits of the scan's and of a tile's wait
@@ -89,6 +90,14 @@ struct ScanState {
 	uint64_t pos, run; // tiles answered, their words
 	uint32_t mx, mask;
 };
+
+// An encode that is lost: no totals (a column that is there has at least one
+// bit in its scheme mask).
+__device__ __forceinline__ void void_info(const EncParams& P) {
+	tile_store(P.info, 0ull);
+	tile_store(P.info + 1, 0ull);
+	tile_store(P.info + 2, 0ull);
+}
 
 // One warp: takes the tiles' reports in order, answers each with its offset
 // and leaves the column's totals in info.  A round reads kScanGroups x 32
@@ -154,7 +163,7 @@ __device__ __forceinline__ uint32_t scan_tiles(const EncParams& P, ScanState& S,
 		if (idle >= P.scan_polls) {
 			if (lane == 0) {
 				atomicOr(P.err, kErrTimeout);
-				P.info[0] = P.info[1] = P.info[2] = 0;
+				void_info(P);
 			}
 			for (uint64_t t = pos + lane; t < P.n_tiles; t += 32u) { tile_store(P.offsets + t, kTileLost); }
 			return 0;
@@ -163,11 +172,23 @@ __device__ __forceinline__ uint32_t scan_tiles(const EncParams& P, ScanState& S,
 	mx   = __reduce_max_sync(0xffffffffu, mx);
 	mask = __reduce_or_sync(0xffffffffu, mask);
 	if (lane == 0) {
-		P.info[0] = run;
-		P.info[1] = mx;
-		P.info[2] = mask;
+		tile_store(P.info, run);
+		tile_store(P.info + 1, mx);
+		tile_store(P.info + 2, mask);
+		__threadfence(); // see tile_lost
+		if (*static_cast<const volatile uint32_t*>(P.lost)) { void_info(P); }
 	}
 	return 0;
+}
+
+// A tile whose wait has run out.  Either the scan, which looks for the mark
+// after it has written its totals, sees it and takes them back, or the totals
+// were there before the mark was, and are taken back here.
+__device__ __forceinline__ void tile_lost(const EncParams& P) {
+	atomicOr(P.err, kErrTimeout);
+	atomicExch(P.lost, 1u);
+	__threadfence();
+	void_info(P);
 }
 
 __device__ __forceinline__ uint32_t bits_of(uint32_t v) { return v ? 32u - __clz(v) : 0u; }
@@ -650,7 +671,7 @@ __device__ __forceinline__ bool encode_tile(const EncParams& P, uint64_t tile, i
 			uint64_t got = 0;
 			for (uint32_t poll = 0; poll < P.tile_polls && got == 0ull; ++poll) { got = tile_load(P.offsets + tile); }
 			if (got == 0ull) {
-				atomicOr(P.err, kErrTimeout);
+				tile_lost(P);
 				got = kTileLost;
 			}
 			T.offset = got;
@@ -671,6 +692,10 @@ __device__ __forceinline__ bool encode_tile(const EncParams& P, uint64_t tile, i
 			P.meta[v] = m;
 		}
 		write_vector(P, v, p, sv, P.out + offset, lane);
+	} else if (live && lane == 0) { // metadata that every decoder refuses
+		fls_vec_meta m {};
+		m.scheme  = FLS_N_SCHEMES;
+		P.meta[v] = m;
 	}
 	__syncthreads(); // T is read before the next tile's
 	return unsure;
@@ -794,7 +819,8 @@ fls_status encode_launch(EncParams& P, uint64_t out_capacity_words, void* d_work
 	P.n_tiles    = (P.n_vec + kEncWarps - 1) / kEncWarps;
 	P.counter    = reinterpret_cast<uint32_t*>(ws);
 	P.n_fallback = reinterpret_cast<unsigned long long*>(ws + 8);
-	P.reports    = reinterpret_cast<uint64_t*>(ws + 16);
+	P.lost       = reinterpret_cast<uint32_t*>(ws + 16);
+	P.reports    = reinterpret_cast<uint64_t*>(ws + 32);
 	P.offsets    = P.reports + P.n_tiles;
 	P.err        = device_error_word(st);
 	const size_t smem = 4u * (kEncWarps * kEncWarpWords + (LEARNED ? sel::WarpNet::kFloats : 0u));
@@ -813,7 +839,7 @@ fls_status encode_launch(EncParams& P, uint64_t out_capacity_words, void* d_work
 			if (dev < 64) { configured |= 1ull << dev; }
 		}
 	}
-	if ((s = cuda_check(cudaMemsetAsync(ws, 0, 16u + 16u * P.n_tiles, st), "cudaMemsetAsync")) != FLS_OK) { return s; }
+	if ((s = cuda_check(cudaMemsetAsync(ws, 0, 32u + 16u * P.n_tiles, st), "cudaMemsetAsync")) != FLS_OK) { return s; }
 	const uint32_t grid = static_cast<uint32_t>(
 	    std::min<uint64_t>(P.n_tiles + 1u, max_ctas ? max_ctas : static_cast<uint64_t>(di.sms) * 3u));
 	enc_kernel<LEARNED><<<grid, kEncWarps * 32, smem, st>>>(P);

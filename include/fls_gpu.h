@@ -178,9 +178,12 @@ fls_status fls_encode_column(const int32_t* values, uint64_t n, const uint8_t* s
  * per-vector scheme is encoded as FOR and flagged in the device error word.
  * d_out holds at least fls_encode_bound_words(n) words; d_meta n_vec entries
  * (both 16-byte aligned); d_info (device uint64[3]) receives the payload words
- * written, the largest vector's words and the scheme mask.  d_workspace holds
- * fls_encode_gpu_workspace_bytes(n) bytes.  Stream-ordered; no reference
- * counterpart (the reference encodes on the host, pack.cpp:29607). */
+ * written, the largest vector's words and the scheme mask.  A mask of 0, which
+ * no column has, is an encode that was lost: a wait on the device ran out
+ * (FLS_ERR_TIMEOUT from fls_check_device_error), the words are not there, and
+ * the vectors without words have metadata that every decoder refuses.
+ * d_workspace holds fls_encode_gpu_workspace_bytes(n) bytes.  Stream-ordered;
+ * no reference counterpart (the reference encodes on the host, pack.cpp:29607). */
 uint64_t   fls_encode_gpu_workspace_bytes(uint64_t n);
 fls_status fls_encode_column_gpu(const int32_t* d_values, uint64_t n, const uint8_t* d_schemes, uint32_t scheme,
                                  uint32_t layout, int round4, uint32_t* d_out, uint64_t out_capacity_words,
