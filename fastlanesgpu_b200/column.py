@@ -271,16 +271,19 @@ class PendingEncode:
     """A GPU encode enqueued without reading its results back: finish() reads
     the encoder's info words (one device-to-host copy) and returns what
     encode_column_learned_gpu returns.  Deferring the read lets many columns
-    be encoded back to back with no host round trip in between."""
+    be encoded back to back with no host round trip in between.  finish() may
+    run under another current stream than the encode's, in any order and from
+    any thread; the column is then ready on that stream."""
 
-    def __init__(self, out, meta, info, schemes, n, layout, compact, defer: bool = True):
+    def __init__(self, out, meta, info, schemes, n, layout, compact, defer: bool = True, stream: int | None = None):
         import torch
         self.out, self.meta, self.info, self.schemes = out, meta, info, schemes
         self.n, self.layout, self.compact = n, layout, compact
         # finish() waits for this encode only, not for what is enqueued after
         # it.  (Not while capturing: finish() then reads in stream order.)
-        self._done = None
+        self._done = self._stream = None
         if defer and not torch.cuda.is_current_stream_capturing():
+            self._stream = stream
             self._done = torch.cuda.Event()
             self._done.record()
 
@@ -292,6 +295,11 @@ class PendingEncode:
                 total, mx, mask, n_fb = _totals(self.info, "fls_encode_learned_gpu")
         else:
             total, mx, mask, n_fb = _totals(self.info, "fls_encode_learned_gpu")
+        if self._stream is not None and self._stream != _lib.stream_handle():
+            # freed memory goes back to the encode's stream: not before this
+            # one is done with it (the copy below, the caller's use)
+            for t in (self.out, self.meta, self.schemes):
+                t.record_stream(torch.cuda.current_stream())
         out = self.out[:max(total, 4)].clone() if self.compact else self.out
         return DeviceEncodedColumn(out, self.meta, self.n, self.layout, total, mx, mask), self.schemes, n_fb
 
@@ -326,11 +334,12 @@ def encode_column_learned_gpu(values, params, threshold: float = 0.9, kappa: flo
     schemes = torch.empty(nv, dtype=torch.uint8, device=dev)
     ws_bytes = int(lib().fls_encode_learned_workspace_bytes(n))
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev)
+    stream = _lib.stream_handle()
     check(lib().fls_encode_learned_gpu(values.data_ptr(), n, params.data_ptr(), threshold, kappa, layout,
                                        out.data_ptr(), bound + 4, meta.data_ptr(), info.data_ptr(), schemes.data_ptr(),
-                                       ws.data_ptr(), ws_bytes, _lib.stream_handle()),
+                                       ws.data_ptr(), ws_bytes, stream),
           "fls_encode_learned_gpu")
-    pending = PendingEncode(out, meta, info, schemes, n, layout, compact, defer)
+    pending = PendingEncode(out, meta, info, schemes, n, layout, compact, defer, stream)
     return pending if defer else pending.finish()
 
 

@@ -2,7 +2,7 @@
 on the device ran out, here because its limit is 0) is an error and its column
 decodes to nothing; deferred encodes finish in any order, on any stream, from
 any thread."""
-import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -10,8 +10,7 @@ import torch
 
 from fastlanesgpu_b200 import LAYOUT_TRANSPOSED, FlsError, _lib, datagen, ops
 from fastlanesgpu_b200 import column as column_module
-from fastlanesgpu_b200.column import (DeviceEncodedColumn, PendingEncode, encode_column_gpu, encode_column_learned_gpu,
-                                      n_vectors)
+from fastlanesgpu_b200.column import (DeviceEncodedColumn, PendingEncode, encode_column_gpu, encode_column_learned_gpu)
 
 MAX_POLLS = 1 << 22
 
@@ -100,4 +99,90 @@ def test_lost_encode(cuda, monkeypatch, polls, n_vec, learned):
     # and afterwards
     monkeypatch.undo()
     assert torch.equal(ops.unpack_global(encode_column_gpu(v, 0), 1)[:n], v)
+    ops.check_device_error()
+
+
+def _check(result, want):
+    (col, schemes, fallback), (wcol, wschemes, wfallback) = result, want
+    assert (col.payload_words, col.desc.max_vec_words, col.desc.scheme_mask, fallback) == \
+        (wcol.payload_words, wcol.desc.max_vec_words, wcol.desc.scheme_mask, wfallback)
+    assert torch.equal(col.data[:col.payload_words], wcol.data[:wcol.payload_words])
+    assert torch.equal(col.meta, wcol.meta) and torch.equal(schemes, wschemes)
+
+
+SIZES = (1, 1024, 5000, 300_000, 77_777, 2_000_001)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("compact", [True, False])
+@pytest.mark.parametrize("finish_on", ["same", "other"])
+def test_deferred_encodes_in_any_order(cuda, compact, finish_on):
+    """Several pending at once, on several streams, finished last to first,
+    under the encode's stream or another one."""
+    params = _params(1)
+    vals = [_values(n, seed=n) for n in SIZES]
+    want = [encode_column_learned_gpu(v, params, compact=compact) for v in vals]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    pending = []
+    for i, v in enumerate(vals):
+        with torch.cuda.stream(streams[i % 3]):
+            pending.append(encode_column_learned_gpu(v, params, compact=compact, defer=True))
+    got = []
+    for i in reversed(range(len(vals))):
+        with torch.cuda.stream(streams[(i + (finish_on == "other")) % 3]):
+            got.insert(0, pending[i].finish())
+    torch.cuda.synchronize()
+    for g, w in zip(got, want):
+        _check(g, w)
+    ops.check_device_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("compact", [True, False])
+def test_finished_column_outlives_its_encode(cuda, compact):
+    """finish() under a busy stream: what the encode allocated is not handed out
+    again while that stream still has to read it."""
+    params, v = _params(2), _values(300_000, seed=9)
+    want = encode_column_learned_gpu(v, params, compact=True)
+    pending = encode_column_learned_gpu(v, params, compact=compact, defer=True)
+    sizes = [pending.out.numel(), pending.meta.numel()]
+    busy = torch.cuda.Stream()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(40_000_000)  # some 20 ms
+        col, schemes, fallback = pending.finish()
+        result = DeviceEncodedColumn(col.data.clone(), col.meta.clone(), col.n_values, col.layout, col.payload_words,
+                                     col.desc.max_vec_words, col.desc.scheme_mask), schemes.clone(), fallback
+    del pending, col, schemes
+    junk = [torch.full((n,), -1, dtype=torch.int32, device="cuda") for n in sizes for _ in range(4)]
+    busy.synchronize()
+    _check(result, want)
+    del junk
+
+
+@pytest.mark.gpu
+def test_deferred_encodes_finished_by_threads(cuda):
+    params = _params(3)
+    vals = [_values(n, seed=n) for n in SIZES]
+    want = [encode_column_learned_gpu(v, params) for v in vals]
+    pending = [encode_column_learned_gpu(v, params, defer=True) for v in vals]
+    got, failed = [None] * len(vals), []
+
+    def work(t):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for i in range(t, len(vals), 2):
+                    got[i] = pending[i].finish()
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(60)
+    assert not failed and not any(t.is_alive() for t in threads)
+    for g, w in zip(got, want):
+        _check(g, w)
     ops.check_device_error()
