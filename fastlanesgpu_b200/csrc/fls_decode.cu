@@ -23,9 +23,18 @@ namespace {
 // 27 -> 23, RLE 37 -> 33, DICT 62 -> 46; to memory, bound by the writes, RLE 41
 // -> 38, DICT 78 -> 57, FOR and DELTA unchanged at 5.5 TB/s; 4 M values, which
 // now reach every SM, 10.2 -> 8.0 to 8.9.
+//
+// A uniform column's vectors lie one after the other at one size, so there a
+// ring's slot holds a tile of several of them, by one copy, and their metadata is
+// the column's.  Sums only: to memory the writes bind.  (134 M values, sum, in
+// tiles of the general pipeline -> vector by vector -> now: DELTA of 2 bits 45.5
+// -> 55.5 -> 35.4 us, of 9 bits 51.3 -> 56.3 -> 39.1; FOR of 4 bits by the general
+// kernel 49.6 -> 60.0 -> 41.2.)
 struct ColumnCfg {
 	DevCol    col;
 	uint64_t  n_vec, n_values;
+	uint64_t  n_items;    // what the ring holds: vectors, or tiles of a uniform column
+	uint32_t  tile;       // vectors per item
 	uint32_t  slots;      // ring depth
 	uint32_t  slot_words; // multiple of 4
 	uint32_t  warps;
@@ -87,7 +96,19 @@ struct ColumnVec {
 	}
 };
 
-template <class Op>
+// Copies tile t of a uniform column; the host has checked that the data covers
+// every vector.
+__device__ __forceinline__ void issue_tile(const ColumnCfg& cfg, uint32_t* slot, uint64_t* bar, uint64_t t,
+                                           uint32_t lane, uint64_t pol) {
+	if (lane == 0) {
+		const uint64_t v0    = t * cfg.tile;
+		const uint32_t bytes = static_cast<uint32_t>(min(static_cast<uint64_t>(cfg.tile), cfg.n_vec - v0)) * cfg.col.vec_words * 4u;
+		dev::mbar_arrive_expect_tx(bar, bytes);
+		if (bytes) { dev::bulk_g2s(slot, cfg.col.data + v0 * cfg.col.vec_words, bytes, bar, pol); }
+	}
+}
+
+template <class Op, bool UNIFORM>
 __global__ void __launch_bounds__(Op::kWarps * 32, 1)
     column_kernel(const __grid_constant__ ColumnCfg cfg, const __grid_constant__ Op op) {
 	extern __shared__ __align__(128) uint32_t smem[];
@@ -97,19 +118,27 @@ __global__ void __launch_bounds__(Op::kWarps * 32, 1)
 	typename Op::State state {};
 	const uint64_t     total = static_cast<uint64_t>(gridDim.x) * cfg.warps;
 	const uint64_t     first = static_cast<uint64_t>(blockIdx.x) * cfg.warps + warp;
-	const uint64_t     n     = first < cfg.n_vec ? (cfg.n_vec - first + total - 1u) / total : 0u;
-	LaneMeta           now = load_window(cfg, first, total, 0, lane), next = load_window(cfg, first, total, 1, lane);
+	const uint64_t     n     = first < cfg.n_items ? (cfg.n_items - first + total - 1u) / total : 0u;
+	LaneMeta           now {}, next {};
+	if constexpr (!UNIFORM) {
+		now  = load_window(cfg, first, total, 0, lane);
+		next = load_window(cfg, first, total, 1, lane);
+	}
 	if (lane < cfg.slots) { dev::mbar_init(bars + lane, 1); }
 	dev::fence_mbar_init();
 	__syncwarp();
 	const uint64_t pol = dev::l2_evict_first_policy();
 	for (uint32_t q = 0; q < cfg.slots && q < n; ++q) {
-		issue_vector(cfg, base + q * cfg.slot_words, bars + q, now, q, lane, pol);
+		if constexpr (UNIFORM) {
+			issue_tile(cfg, base + q * cfg.slot_words, bars + q, first + q * total, lane, pol);
+		} else {
+			issue_vector(cfg, base + q * cfg.slot_words, bars + q, now, q, lane, pol);
+		}
 	}
 	uint32_t slot = 0, phase = 0;
 	for (uint64_t q = 0; q < n; ++q) {
 		const uint32_t j = static_cast<uint32_t>(q) & 31u;
-		if (j == 0 && q != 0) {
+		if (!UNIFORM && j == 0 && q != 0) {
 			now  = next;
 			next = load_window(cfg, first, total, (q >> 5) + 1u, lane);
 		}
@@ -122,22 +151,36 @@ __global__ void __launch_bounds__(Op::kWarps * 32, 1)
 			}
 			return;
 		}
-		const uint32_t packed = __shfl_sync(0xffffffffu, now.packed, j);
-		ColumnVec      cv;
-		cv.vi.base   = static_cast<int32_t>(__shfl_sync(0xffffffffu, now.base, j));
-		cv.vi.scheme = packed & 0xffu;
-		cv.vi.bw     = (packed >> 8) & 0xffu;
-		cv.vi.aux    = packed >> 16;
-		cv.s         = base + slot * cfg.slot_words;
-		cv.dict      = base + cfg.dict_off;
-		cv.extra     = base + cfg.extra_off;
-		cv.v         = first + q * total;
-		if (cv.vi.scheme != kBadScheme) { op.process(state, cv, lane, cfg); }
+		ColumnVec cv;
+		cv.s     = base + slot * cfg.slot_words;
+		cv.dict  = base + cfg.dict_off;
+		cv.extra = base + cfg.extra_off;
+		if constexpr (UNIFORM) {
+			cv.vi.base   = cfg.col.base;
+			cv.vi.scheme = cfg.col.scheme;
+			cv.vi.bw     = cfg.col.bw;
+			cv.vi.aux    = 0;
+			cv.v         = (first + q * total) * cfg.tile;
+			const uint64_t end = min(cv.v + cfg.tile, cfg.n_vec);
+			for (; cv.v < end; ++cv.v, cv.s += cfg.col.vec_words) { op.process(state, cv, lane, cfg); }
+		} else {
+			const uint32_t packed = __shfl_sync(0xffffffffu, now.packed, j);
+			cv.vi.base   = static_cast<int32_t>(__shfl_sync(0xffffffffu, now.base, j));
+			cv.vi.scheme = packed & 0xffu;
+			cv.vi.bw     = (packed >> 8) & 0xffu;
+			cv.vi.aux    = packed >> 16;
+			cv.v         = first + q * total;
+			if (cv.vi.scheme != kBadScheme) { op.process(state, cv, lane, cfg); }
+		}
 		__syncwarp();
 		if (q + cfg.slots < n) {
 			dev::fence_proxy_async_smem();
-			const uint32_t ahead = j + cfg.slots; // below 64
-			issue_vector(cfg, base + slot * cfg.slot_words, bars + slot, ahead < 32u ? now : next, ahead & 31u, lane, pol);
+			if constexpr (UNIFORM) {
+				issue_tile(cfg, base + slot * cfg.slot_words, bars + slot, first + (q + cfg.slots) * total, lane, pol);
+			} else {
+				const uint32_t ahead = j + cfg.slots; // below 64
+				issue_vector(cfg, base + slot * cfg.slot_words, bars + slot, ahead < 32u ? now : next, ahead & 31u, lane, pol);
+			}
 		}
 		if (++slot == cfg.slots) {
 			slot = 0;
@@ -154,9 +197,11 @@ __global__ void __launch_bounds__(Op::kWarps * 32, 1)
 // past that the reads in flight only disturb the writes (67 M values to
 // memory: DELTA 59.0 us at 4 KB a warp, 61.7 at 6 KB; in original order 59.4
 // at 6 KB, 59.8 at 4 and 61.0 at 8; FOR of mixed widths 68.5, 69.3 at 12).  A
-// column of fewer vectors than warps spreads over the SMs.
-template <class Op>
-fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_words, cudaStream_t stream) {
+// column of fewer items than warps spreads over the SMs.  A uniform column's
+// tiles are as long as a tile of the launch configuration, or shorter so that
+// every warp gets four.
+template <class Op, bool UNIFORM>
+fls_status launch_column_as(const fls_column& col, const Op& op, uint32_t extra_words, cudaStream_t stream) {
 	ColumnCfg  cfg {};
 	DeviceInfo di;
 	fls_status s = device_info(di);
@@ -169,20 +214,28 @@ fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_wor
 	cfg.n_values = col.n_values;
 	cfg.n_vec    = (col.n_values + 1023u) / 1024u;
 	const auto round4 = [](uint32_t w) { return (w + 3u) & ~3u; };
-	cfg.slot_words    = round4(cfg.col.slot_words);
-	const uint32_t flight = stages * tile_bytes / op.flight_share();
-	const uint32_t want   = std::max<uint32_t>(1u, flight / std::max<uint32_t>(4u * cfg.slot_words, 256u));
 	const uint32_t fixed = kSlotSlackWords + (cfg.has_dict ? kDictWords : 0u) + round4(extra_words) + 2u * kMaxSlots;
 	const uint32_t avail = static_cast<uint32_t>(di.max_smem) / 4u;
+	cfg.tile             = 1;
+	if (UNIFORM) { // two tiles of all warps fit
+		const uint64_t all   = static_cast<uint64_t>(di.sms) * ctas * warps;
+		const uint32_t words = std::min<uint32_t>(tile_bytes / 4u, (avail / warps - fixed) / 2u);
+		cfg.tile             = std::max<uint32_t>(1u, std::min<uint32_t>(kMaxTile, words / std::max<uint32_t>(cfg.col.vec_words, 32u)));
+		while (cfg.tile > 1 && cfg.n_vec / cfg.tile < 4u * all) { cfg.tile /= 2u; }
+	}
+	cfg.n_items           = (cfg.n_vec + cfg.tile - 1u) / cfg.tile;
+	cfg.slot_words        = round4(cfg.tile * cfg.col.slot_words);
+	const uint32_t flight = stages * tile_bytes / op.flight_share();
+	const uint32_t want   = std::max<uint32_t>(1u, flight / std::max<uint32_t>(4u * cfg.slot_words, 256u));
 	const auto     fits  = [&](uint32_t w, uint32_t slots) { return w * (slots * cfg.slot_words + fixed) <= avail; };
 	while (warps > 1 && !fits(warps, 2)) { --warps; }
 	if (!fits(warps, 1)) { return set_error(FLS_ERR_CAPACITY, "vectors too large for shared-memory staging"); }
 	cfg.slots = std::min<uint32_t>(std::max<uint32_t>(want, 2u), kMaxSlots);
 	while (cfg.slots > 1 && !fits(warps, cfg.slots)) { --cfg.slots; }
-	uint64_t grid = std::min<uint64_t>((cfg.n_vec + warps - 1u) / warps, static_cast<uint64_t>(di.sms) * ctas);
+	uint64_t grid = std::min<uint64_t>((cfg.n_items + warps - 1u) / warps, static_cast<uint64_t>(di.sms) * ctas);
 	if (grid < static_cast<uint64_t>(di.sms)) {
-		grid  = std::min<uint64_t>(cfg.n_vec, static_cast<uint64_t>(di.sms));
-		warps = static_cast<uint32_t>((cfg.n_vec + grid - 1u) / grid);
+		grid  = std::min<uint64_t>(cfg.n_items, static_cast<uint64_t>(di.sms));
+		warps = static_cast<uint32_t>((cfg.n_items + grid - 1u) / grid);
 	}
 	cfg.warps      = warps;
 	cfg.dict_off   = cfg.slots * cfg.slot_words + kSlotSlackWords;
@@ -197,15 +250,23 @@ fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_wor
 		cudaGetDevice(&dev);
 		std::lock_guard<std::mutex> lk(mu);
 		if (dev >= 64 || !(configured & (1ull << dev))) {
-			s = cuda_check(cudaFuncSetAttribute(column_kernel<Op>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem),
+			s = cuda_check(cudaFuncSetAttribute(column_kernel<Op, UNIFORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem),
 			               "cudaFuncSetAttribute");
 			if (s != FLS_OK) { return s; }
 			if (dev < 64) { configured |= 1ull << dev; }
 		}
 	}
-	column_kernel<Op><<<static_cast<uint32_t>(grid), 32u * warps, 4ull * cfg.warp_words * warps, stream>>>(cfg, op);
+	column_kernel<Op, UNIFORM><<<static_cast<uint32_t>(grid), 32u * warps, 4ull * cfg.warp_words * warps, stream>>>(cfg, op);
 	count_launch();
 	return cuda_check(cudaGetLastError(), "column_kernel launch");
+}
+
+template <class Op>
+fls_status launch_column(const fls_column& col, const Op& op, uint32_t extra_words, cudaStream_t stream) {
+	if constexpr (Op::kTiles) {
+		if (!col.meta) { return launch_column_as<Op, true>(col, op, extra_words, stream); }
+	}
+	return launch_column_as<Op, false>(col, op, extra_words, stream);
 }
 
 // -------------------------------------------------------------- operators
@@ -225,6 +286,7 @@ struct NoState {};
 // 46.3).
 struct DecodeOp {
 	static constexpr uint32_t kWarps = 16;
+	static constexpr bool     kTiles = false; // bound by the writes: no faster in tiles
 	uint32_t flight_share() const { return original ? 2u : 3u; }
 	using State = NoState;
 	uint32_t* out;
@@ -278,6 +340,7 @@ struct AccState {
 // atomic per warp at the end.
 struct DecodeSumOp {
 	static constexpr uint32_t kWarps = 16;
+	static constexpr bool     kTiles = true;
 	uint32_t flight_share() const { return 1u; }
 	using State = AccState;
 	unsigned long long* sum;
@@ -431,6 +494,7 @@ struct SchemeSumOp {
 	// 50 M values, kernel at 16, 24 and 32 warps (us): DELTA 20.2, 18.1, 18.4; RLE
 	// 29.7, 27.3, 26.5; DICT 43.5, 39.9, 39.9.
 	static constexpr uint32_t kWarps = 24;
+	static constexpr bool     kTiles = SCHEME == FLS_SCHEME_DELTA; // the one that a uniform column may have
 	uint32_t flight_share() const { return 1u; }
 	using State = AccState;
 	unsigned long long* sum;
@@ -484,11 +548,9 @@ struct SchemeSumOp {
 	}
 };
 
-// The single scheme of a per-vector column that has a specialised sum, or
-// FLS_N_SCHEMES.
+// The single scheme of a column, if it has a specialised sum, or FLS_N_SCHEMES.
 uint32_t single_scheme(const fls_column& c) {
-	if (!c.meta) { return FLS_N_SCHEMES; }
-	const uint32_t m = c.scheme_mask;
+	const uint32_t m = c.meta ? c.scheme_mask : 1u << c.scheme;
 	if (m == (1u << FLS_SCHEME_DELTA)) { return FLS_SCHEME_DELTA; }
 	if (m == (1u << FLS_SCHEME_RLE)) { return FLS_SCHEME_RLE; }
 	if (m == (1u << FLS_SCHEME_DICT)) { return FLS_SCHEME_DICT; }

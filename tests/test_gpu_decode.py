@@ -223,3 +223,29 @@ def test_original_order_into_any_alignment(cuda, shift, scheme):
     got = buf.cpu().numpy()
     assert np.array_equal(got[shift:shift + 6 * 1024], _pad(v))
     assert np.all(got[:shift] == -7) and np.all(got[shift + 6 * 1024:] == -7)
+
+
+@pytest.mark.parametrize("n_vec", [1, 5, 148 * 8 - 1, 148 * 8 + 1, 148 * 16 + 9, 148 * 128 + 3])
+@pytest.mark.parametrize("scheme,bw", [(0, 0), (0, 1), (0, 13), (0, 32), (1, 0), (1, 3), (1, 22), (1, 23), (1, 32)])
+def test_uniform_sum_in_tiles(cuda, n_vec, scheme, bw):
+    """Sums of uniform columns by tiles of several vectors, from one vector per
+    tile to the longest, with a short last tile and a partial last vector; FOR
+    by the general kernel."""
+    import torch
+    from fastlanesgpu_b200.column import DeviceUniformColumn
+    n = n_vec * 1024 - 9
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n_vec + bw)
+    words = max(4, n_vec * (32 * bw + 32 * scheme))
+    data = torch.randint(-2**31, 2**31, (words,), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    col = DeviceUniformColumn(data, n, bw, base=-3 if scheme == 0 else 0, scheme=scheme, layout=1)
+    ops.set_tuning(1, int(scheme == 1))
+    try:
+        want = int((ops.unpack_global(col, ORDER_ORIGINAL)[:n].long() & 0xFFFFFFFF).sum())
+        for config in ((0, 0, 0, 0), (1, 2, 1, 65536), (1, 4, 1, 2048), (5, 2, 2, 6144)):
+            ops.set_launch_config(*config)
+            assert int(ops.query_aggregate(col).cpu()[0]) == want, config
+        ops.check_device_error()
+    finally:
+        ops.set_launch_config()
+        ops.set_tuning(1, 1)
