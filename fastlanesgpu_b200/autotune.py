@@ -19,7 +19,7 @@ import os
 from . import ops
 
 DEFAULT_SPACE = {
-    "warps": [8, 16],
+    "warps": [0, 8, 16],  # 0: the library's choice, more than 16 for some kernels
     "stages": [2, 3],
     "tile_bytes": [2048, 6144, 16384],
     "sparse_rows": [2, 4, 8],

@@ -546,8 +546,14 @@ fls_status fls_crystal_q21_probe(const int32_t* suppkey, uint32_t supp_bw, const
  * pipeline stages per warp, CTAs per SM and the target bytes of one staged
  * tile of consecutive vectors (0 = library default for each).  Used by the
  * autotuner; applies to subsequent calls from all threads.  Until warps are
- * set here, the specialised join + group-by kernels (FLS_TUNE_JIT) use up to
- * 20 warps per CTA where shared memory allows, every other kernel 16. */
+ * set here, the specialised join + group-by kernels (FLS_TUNE_JIT) and the sums
+ * of columns whose vectors all have one scheme (DELTA, RLE or DICT) use up to 24
+ * warps per CTA where shared memory allows, every other kernel 16, which is
+ * what fls_get_launch_config reports then.  fls_decode_u32 and
+ * fls_decode_sum_u32 keep a ring of vectors per warp (tiles of vectors for the
+ * sum of a uniform column) instead of a fixed number of stages: stages x
+ * tile_bytes bounds the bytes that a warp has in flight (a third of it, or half
+ * in original order, where the values are written out), in 2 to 16 slots. */
 fls_status fls_set_launch_config(uint32_t warps_per_cta, uint32_t stages, uint32_t ctas_per_sm, uint32_t tile_bytes);
 fls_status fls_get_launch_config(uint32_t* warps_per_cta, uint32_t* stages, uint32_t* ctas_per_sm,
                                  uint32_t* tile_bytes);

@@ -81,3 +81,19 @@ def test_reset_restores_every_default():
         assert (ops.get_launch_config(), [ops.get_tuning(p) for p in (0, 2, 3, 4, 5)]) == before
     finally:
         autotune.reset()
+
+
+def test_default_space_times_and_keeps_the_library_default(monkeypatch):
+    """The library picks the warps by kernel until they are set, so that choice
+    is a candidate of its own, and winning leaves it in place."""
+    from fastlanesgpu_b200 import ops
+    chosen = []
+    real = ops.set_launch_config
+    monkeypatch.setattr(ops, "set_launch_config", lambda *a: (chosen.append(a), real(*a)))
+    monkeypatch.setattr(autotune, "time_ms", lambda fn, warmup=3, iters=10: 1.0 + (chosen[-1][0] != 0))
+    try:
+        best = autotune.tune("t", lambda: None, use_cache=False)
+        assert best["config"]["warps"] == 0 and chosen[-1][0] == 0
+        assert {c["warps"] for c in best["candidates"]} >= {0, 8, 16}
+    finally:
+        autotune.reset()
