@@ -58,7 +58,6 @@ struct StageCfg {
 	uint32_t  warps;           // W
 	uint32_t  warp_smem_words; // per-warp region (multiple of 4)
 	uint32_t  dict_off;        // per-warp dictionary scratch (words)
-	uint32_t  extra_off;       // per-warp operator scratch (words)
 	uint32_t  info_off;        // per-warp vector info: uint4 per (stage, vector, column)
 	uint32_t  bar_off;         // per-warp mbarriers (uint64 per stage)
 	uint32_t  cta_extra_off;   // CTA-level scratch after all warp regions (words)
@@ -88,7 +87,6 @@ struct WarpStage {
 	}
 	__device__ uint64_t* bar(uint32_t st) const { return reinterpret_cast<uint64_t*>(base + cfg->bar_off) + st; }
 	__device__ uint32_t* dict() const { return base + cfg->dict_off; }
-	__device__ uint32_t* extra() const { return base + cfg->extra_off; }
 };
 
 // Issues the bulk copies of tile t into stage st.  All lanes participate in
@@ -373,10 +371,10 @@ uint64_t jit_probe_workspace_bytes(const fls_join_groupby_desc* desc);
 fls_status jit_decode(const fls_column* col, int mode, uint32_t* d_out, uint64_t* d_sum, cudaStream_t stream,
                       bool& used);
 
-// Lays out shared memory for a set of columns; extra_words per warp and
-// cta_words per CTA are operator-specific scratch.
-fls_status plan_stages(const fls_column* cols, uint32_t n_cols, uint32_t extra_words, uint32_t cta_words,
-                       StageCfg& cfg, uint32_t& grid, uint32_t& threads, size_t& smem_bytes);
+// Lays out shared memory for a set of columns; cta_words per CTA are
+// operator-specific scratch.
+fls_status plan_stages(const fls_column* cols, uint32_t n_cols, uint32_t cta_words, StageCfg& cfg, uint32_t& grid,
+                       uint32_t& threads, size_t& smem_bytes);
 
 template <class Op>
 fls_status launch_staged(const StageCfg& cfg, const Op& op, uint32_t grid, uint32_t threads, size_t smem,

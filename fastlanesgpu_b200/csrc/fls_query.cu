@@ -722,7 +722,7 @@ fls_status fls_query_filter_agg(const fls_filter_agg_desc* desc, int64_t* d_resu
 	StageCfg cfg;
 	uint32_t grid, threads;
 	size_t   smem;
-	s = plan_stages(desc->cols, desc->n_cols, 0u, 0u, cfg, grid, threads, smem);
+	s = plan_stages(desc->cols, desc->n_cols, 0u, cfg, grid, threads, smem);
 	if (s != FLS_OK) { return s; }
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 	if ((s = cuda_check(cudaMemsetAsync(d_result, 0, sizeof(int64_t), st), "cudaMemsetAsync")) != FLS_OK) { return s; }
@@ -878,7 +878,7 @@ fls_status fls_query_join_groupby_ws(const fls_join_groupby_desc* desc, int32_t*
 	StageCfg cfg;
 	uint32_t grid, threads;
 	size_t   smem;
-	s = plan_stages(desc->cols, desc->n_cols, 0u, cta_words, cfg, grid, threads, smem);
+	s = plan_stages(desc->cols, desc->n_cols, cta_words, cfg, grid, threads, smem);
 	if (s != FLS_OK) { return s; }
 	cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 	s = cuda_check(cudaMemsetAsync(d_res, 0,

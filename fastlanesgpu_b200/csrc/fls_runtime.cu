@@ -182,8 +182,8 @@ bool needs_dict(const fls_column& c) {
 }
 } // namespace
 
-fls_status plan_stages(const fls_column* cols, uint32_t n_cols, uint32_t extra_words, uint32_t cta_words,
-                       StageCfg& cfg, uint32_t& grid, uint32_t& threads, size_t& smem_bytes) {
+fls_status plan_stages(const fls_column* cols, uint32_t n_cols, uint32_t cta_words, StageCfg& cfg, uint32_t& grid,
+                       uint32_t& threads, size_t& smem_bytes) {
 	if (!cols || n_cols == 0 || n_cols > kMaxCols) { return set_error(FLS_ERR_INVALID_ARG, "1..8 columns per query"); }
 	DeviceInfo di;
 	fls_status s = device_info(di);
@@ -230,8 +230,6 @@ fls_status plan_stages(const fls_column* cols, uint32_t n_cols, uint32_t extra_w
 		uint32_t w   = S * cfg.stage_words + kSlotSlackWords;
 		cfg.dict_off = w;
 		w += dict ? kDictWords : 0u;
-		cfg.extra_off = w;
-		w += round4(extra_words);
 		cfg.info_off = w;
 		w += 4u * S * k * n_cols;
 		cfg.bar_off = w;
