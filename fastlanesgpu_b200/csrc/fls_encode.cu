@@ -37,7 +37,11 @@ constexpr uint32_t kNetWords     = sel::kPadded + sel::kBuckets / 4u; // offset 
 static_assert(kEncWarpWords % 4 == 0 && kEncWarpWords >= kNetWords + sel::WarpNet::kScratch, "the warp's words");
 constexpr uint32_t kKeyedBits    = 22;               // widest range whose sort keys carry the value's index
 constexpr uint32_t kPollLimit   = 1u << 22;          // bounded waits on other tiles (each poll is an L2 round trip)
-constexpr uint32_t kAloneRounds = 64;                // idle rounds after which the scan looks whether any tile is taken
+// Idle rounds (some 5 ms) after which the scan looks whether any tile is taken:
+// encodes that share the GPU with others wait for places for a while, and a tile
+// by the scanning CTA holds up the answers to all others (64 columns on four
+// streams, whole calls: 4.4 ms at 64 rounds, 4.2 so).
+constexpr uint32_t kAloneRounds = 1u << 13;
 
 struct EncParams {
 	const int32_t* values;
