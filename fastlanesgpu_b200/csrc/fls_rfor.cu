@@ -26,10 +26,11 @@
 // A tile whose block is inconsistent is skipped and flagged, never read past
 // its stream.
 //
-// Bounded by integer issue (70 % of it active).  16.8 M values of geometric
-// runs (mean 16), kernel, against contiguous chunks of runs per lane, one
-// position per lane and row and the sum over expanded positions: to memory
-// 20.7 -> 19.3 us, sum 20.5 -> 13.1.
+// Bounded by integer issue (68 % of it active, 430 warp instructions per tile to
+// memory) and, in the rest, by reads and chains of shuffles that too few warps
+// cover.  16.8 M values of geometric runs (mean 16), whole call, against
+// contiguous chunks of runs per lane, one position per lane and row and the sum
+// over expanded positions: to memory 22.7 -> 20.7 us, sum 22.8 -> 14.5.
 #include "fls_pipeline.cuh"
 
 namespace fls {
@@ -55,16 +56,15 @@ __device__ __forceinline__ uint32_t packed_words(uint32_t count, uint32_t bw) {
 // k*bw, LSB first): word row i of bw words holds fields 32 i .. 32 i + 31.
 // Never reads past the block's last packed word.
 struct LaneFields {
-	const uint32_t *block, *p;
+	const uint32_t* p;
 	uint32_t        bw, sh, mask, next;
-	__device__ __forceinline__ LaneFields(const uint32_t* words, uint32_t width, uint32_t lane) {
+	__device__ __forceinline__ LaneFields(const uint32_t* block, uint32_t width, uint32_t lane) {
 		const uint32_t bit = lane * width;
-		block = words;
-		p     = words + (bit >> 5);
-		bw    = width;
-		sh    = bit & 31u;
-		mask  = width >= 32 ? 0xffffffffu : ((1u << width) - 1u);
-		next  = sh + width > 32u ? 1u : 0u; // without a second word the first is read twice and masked off
+		p    = block + (bit >> 5);
+		bw   = width;
+		sh   = bit & 31u;
+		mask = width >= 32 ? 0xffffffffu : ((1u << width) - 1u);
+		next = sh + width > 32u ? 1u : 0u; // without a second word the first is read twice and masked off
 	}
 	// Row i's field; the caller has checked that it is one of the block's.
 	__device__ __forceinline__ uint32_t get(uint32_t i) const {
@@ -72,8 +72,9 @@ struct LaneFields {
 		const uint32_t* q = p + i * bw;
 		return __funnelshift_r(__ldg(q), __ldg(q + next), sh) & mask;
 	}
-	// Field k, whichever lane's it is (a block of width 0 still has one word).
-	__device__ __forceinline__ uint32_t any(uint32_t k) const {
+	__device__ __forceinline__ const uint32_t* block(uint32_t lane) const { return p - ((lane * bw) >> 5); }
+	// Field k of the block, whichever lane's it is (a block of width 0 still has one word).
+	__device__ __forceinline__ uint32_t any(const uint32_t* block, uint32_t k) const {
 		const uint32_t  bit = k * bw, s = bit & 31u;
 		const uint32_t* q = block + (bit >> 5);
 		return __funnelshift_r(__ldg(q), s + bw > 32u ? __ldg(q + 1) : 0u, s) & mask;
@@ -144,7 +145,7 @@ __device__ __forceinline__ TileHead load_head(const RforParams& P, uint64_t t) {
 // memory per 32 runs, and their starts, close together, meet in a word or two,
 // one atomic after the other (16.8 M values, whole call, 32 at a time -> this:
 // to memory, runs of mean 2 57 -> 37 and 4 37 -> 27 us; 1 stays at 104, bound by
-// the bank conflicts of chunks of 16; sums 64 -> 53, 47 -> 41 and 31 -> 27 with
+// the bank conflicts of chunks of 16; sums 64 -> 51, 48 -> 34 and 31 -> 23 with
 // the whole tiles' sums below).  `total`: the positions covered; SUM (of the
 // positions below `live`) into part.  False where a run has length 0 or passes
 // the tile: nothing that counts is done then.
@@ -153,12 +154,13 @@ template <bool SUM>
 __device__ __forceinline__ bool many_runs(const LaneFields& vf, const LaneFields& rf, uint32_t vmin, uint32_t rmin,
                                           uint32_t cnt, uint32_t live, uint32_t* vals, uint16_t* lens, uint2* words,
                                           uint32_t lane, uint32_t& total, unsigned long long& part) {
+	const uint32_t *vb = vf.block(lane), *rb = rf.block(lane);
 	const uint32_t chunk = (cnt + 31u) >> 5, k0 = min(cnt, lane * chunk), k1 = min(cnt, k0 + chunk);
 	uint32_t       own = 0, most = 0; // most: the largest length minus one
 	for (uint32_t k = k0; k < k1; ++k) {
-		const uint32_t l = rmin + rf.any(k);
+		const uint32_t l = rmin + rf.any(rb, k);
 		if constexpr (!SUM) {
-			vals[k] = vmin + vf.any(k);
+			vals[k] = vmin + vf.any(vb, k);
 			lens[k] = static_cast<uint16_t>(l);
 		}
 		most = max(most, l - 1u);
@@ -179,8 +181,8 @@ __device__ __forceinline__ bool many_runs(const LaneFields& vf, const LaneFields
 		uint32_t pos = incl - own;
 		for (uint32_t k = k0; k < k1; ++k) {
 			if constexpr (SUM) {
-				const uint32_t l = rmin + rf.any(k);
-				part += static_cast<unsigned long long>(vmin + vf.any(k)) * (min(pos + l, live) - min(pos, live));
+				const uint32_t l = rmin + rf.any(rb, k);
+				part += static_cast<unsigned long long>(vmin + vf.any(vb, k)) * (min(pos + l, live) - min(pos, live));
 				pos += l;
 			} else { // each lane reads back its own lengths
 				atomicOr(&words[pos >> 5].x, 1u << (pos & 31u));
@@ -227,10 +229,11 @@ __global__ void __launch_bounds__(kRforWarps * 32, SUM ? 6 : 5) rfor_kernel(cons
 		bool               fits  = true, grouped = true;
 		if (SUM && live == kTile) {
 			// A whole tile's sum needs no positions: no scan, every read
-			// independent of the one before.
+			// independent of the one before.  (Unrolled it is slower, 34 -> 41
+			// us at runs of mean 2.)
 			grouped        = false;
 			uint32_t cover = 0;
-#pragma unroll 4
+#pragma unroll 1
 			for (uint32_t i = 0; 32u * i < cnt; ++i) {
 				if (32u * i + lane < cnt) {
 					const uint32_t l = rmin + rf.get(i), v = vmin + vf.get(i);
