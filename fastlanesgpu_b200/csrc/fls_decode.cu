@@ -196,7 +196,8 @@ __global__ void __launch_bounds__(Op::kWarps * 32, 1)
 // of them where every vector is also written out (half in original order):
 // past that the reads in flight only disturb the writes (67 M values to
 // memory: DELTA 59.0 us at 4 KB a warp, 61.7 at 6 KB; in original order 59.4
-// at 6 KB, 59.8 at 4 and 61.0 at 8; FOR of mixed widths 68.5, 69.3 at 12).  A
+// at 6 KB, 59.8 at 4 and 61.0 at 8; FOR of mixed widths 68.5, 69.3 at 12; at 1 to
+// 8 M values a warp has few vectors and the share makes no difference).  A
 // column of fewer items than warps spreads over the SMs.  A uniform column's
 // tiles are as long as a tile of the launch configuration, or shorter so that
 // every warp gets four.
@@ -492,7 +493,9 @@ __device__ __forceinline__ unsigned long long dict_lane_sum(const uint32_t* __re
 template <uint32_t SCHEME>
 struct SchemeSumOp {
 	// 50 M values, kernel at 16, 24 and 32 warps (us): DELTA 20.2, 18.1, 18.4; RLE
-	// 29.7, 27.3, 26.5; DICT 43.5, 39.9, 39.9.
+	// 29.7, 27.3, 26.5; DICT 43.5, 39.9, 39.9.  Short columns, whole call at 16 and
+	// 24: DICT 1 M 8.3, 8.3, 4 M (two vectors for some warps of 24) 10.4, 12.3, 8 M
+	// 14.5, 14.3; RLE 4 M 8.3, 9.9, 8 M 10.4, 10.6; DELTA 4 M 8.3, 8.3.
 	static constexpr uint32_t kWarps = 24;
 	static constexpr bool     kTiles = SCHEME == FLS_SCHEME_DELTA; // the one that a uniform column may have
 	uint32_t flight_share() const { return 1u; }

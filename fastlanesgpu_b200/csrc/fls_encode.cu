@@ -733,15 +733,15 @@ __device__ __forceinline__ uint32_t encode_alone(const EncParams& P, uint32_t ti
 // in columns of few rounds, by the round trip of a tile's offset, 2-4 us.
 // 1568 words per warp let three CTAs (24 warps) share an SM.  Against separate
 // plan, scan and write kernels, which read and sorted everything twice, whole
-// encoder calls took (us, before -> after; about 60 of each are the call's
-// host side and its read-back): 6 M values DICT 437 -> 120, 33.5 M values FOR
+// encoder calls took (us, before -> after; about 40 of each are the call's
+// host side and its read-back): 6 M values DICT 437 -> 104, 33.5 M values FOR
 // 186 -> 120, DELTA 185 -> 118, RLE 185 -> 145, DICT 1920 -> 315.
 //
 // LEARNED: a warp first takes its vector's statistics and runs the network on
 // them (fls_selector.cuh), so the values are still read once and the column
 // takes one launch instead of eight (four columns of 8.4 M values: statistics
 // 20, network 21, choice 6, plan 18, scans 10, write 18-41 us each -> 40-50;
-// the whole call 576 -> 387 us).
+// the whole call 576 -> 325 us).
 template <bool LEARNED>
 __global__ void __launch_bounds__(kEncWarps * 32, 3) enc_kernel(const __grid_constant__ EncParams P) {
 	extern __shared__ __align__(16) int32_t esmem[];
